@@ -7,9 +7,9 @@
 // reference (cuda/ccl_uf.cu:64-157, UF_local / UF_global / UF_final) uses the same
 // min-index rule with atomicMin.  This implementation keeps that rule (so labels are
 // bit-identical) with its own schedule:
-//   1. ccl_local: 32x32 tile per CTA; horizontal runs from warp ballots, union-find on run
-//      contacts in shared memory with atomicMin hooking; writes the tile-local root's global
-//      index, lists the local roots and (optionally) their areas.
+//   1. ccl_local: 32x32 tile per warp; rows as bit masks from ballots, runs joined by pointer
+//      jumping and (for the few that touch two runs above) unions in shared memory; writes the
+//      tile-local root's global index, lists the local roots and (optionally) their areas.
 //   2. ccl_merge: one warp per tile edge joins runs that touch across the edge (global
 //      atomicMin hooking; a failed hook retries with the new parent).
 //   3. ccl_flatten_roots: every local root points directly at its global root and passes its
@@ -50,19 +50,27 @@ __device__ __forceinline__ bool joins_diagonally(uint32_t c) {
   else if constexpr (CONN == kConnFg8Bg4) return c == 1u;
   else return c == 2u;
 }
-constexpr int kThreads = 256;            // threads per labelling tile (32 columns x 8 warps)
-constexpr int kRows = kTile / (kThreads / 32);  // tile rows per thread (consecutive)
+constexpr int kLocalWarps = 4;  // labelling tiles (one warp each) per CTA of ccl_local
 
-// Root of x in a shared-memory forest, halving the path on the way (every node on it is
-// re-pointed to its grandparent; a concurrent hook of a root is never overwritten because
-// roots are not written here).
+// Tile-local forest of one warp (shared memory, 1024 words).  Node i = 32 * row + column; its
+// word sits at s[i ^ (i >> 5)], so the same column of 32 rows lies in 32 banks.  A word holds the
+// parent in its low 10 bits; the area of a root is added above bit 16 once the unions are done.
+constexpr int kNodeMask = kTile * kTile - 1;
+__device__ __forceinline__ int node_at(int i) { return i ^ (i >> 5); }
+
+// Root of x, halving the path on the way (every node on it is re-pointed to its grandparent; a
+// concurrent hook of a root is never overwritten because roots are not written here).  FINAL: the
+// unions are done and other lanes write final roots into these words, so a re-pointing is an
+// atomicMin (a parent only ever moves to a smaller node, and the root is the smallest of all).
+template <bool FINAL = false>
 __device__ __forceinline__ int s_find(volatile int* s, int x) {
   for (;;) {
-    const int p = s[x];
+    const int p = s[node_at(x)] & kNodeMask;
     if (p == x) return x;
-    const int g = s[p];
+    const int g = s[node_at(p)] & kNodeMask;
     if (g == p) return p;
-    s[x] = g;
+    if (FINAL) atomicMin((int*)&s[node_at(x)], g);
+    else s[node_at(x)] = g;
     x = g;
   }
 }
@@ -77,7 +85,7 @@ __device__ __forceinline__ void s_union(int* s, int a, int b) {
       a = b;
       b = t;
     }
-    const int old = atomicMin(&s[a], b);
+    const int old = atomicMin(&s[node_at(a)], b);
     if (old == a) return;
     a = old;
   }
@@ -169,145 +177,269 @@ struct class_type<Cls, std::void_t<typename Cls::class_t>> {
   using type = typename Cls::class_t;
 };
 
-// Each warp owns kRows consecutive tile rows (lane = column) and joins them top-down, so a
-// row's runs hook straight onto the root already found for the row above; only the four
-// warps' blocks meet concurrently, which keeps the trees (and every later find) shallow.  Runs of equal class along a row are found with a
-// ballot and start out joined (label = run start), so unions are only needed where runs of
-// adjacent rows touch: at a pixel that starts its run or sits under the start of a run above
-// (and, for 8-connectivity, diagonally past the two ends of the run).  That is one union per
-// touching pair of runs instead of one per pixel pair.  One CTA per labelling tile (1-D grid
-// over the tiles of all images).
+// What a classifier's values can be (`Cls::kKind`): any value, background 0 or class 1, class 1
+// or class 2 (no background inside the image), or class 0 / 1 given as 32 pixels of a row at once
+// (row_bits).
+enum ClassKind { kAnyClass, kOneClass, kTwoClasses, kRowBits };
+
+// The rows of a labelling tile as bit masks (bit = column), lane = row: the foreground, the run
+// starts, and the pixels at which a union with the row above is due -- straight up, up-left, up-right.
+struct RowMasks {
+  unsigned fg, start, up, ul, ur;
+};
+
+__device__ __forceinline__ unsigned above(unsigned m, int lane) {
+  const unsigned u = __shfl_up_sync(NSGB_FULL, m, 1);
+  return lane ? u : 0u;
+}
+
+// One class (mask m of this lane's row): a pair of touching runs of adjacent rows is joined once,
+// at the first column of their overlap, or diagonally past an end of the lower run where the
+// pixel above that end is not of the class.
+__device__ __forceinline__ void class_masks(unsigned m, bool diag, int lane, RowMasks& k) {
+  const unsigned u = above(m, lane), st = m & ~(m << 1), c = m & u;
+  k.fg |= m;
+  k.start |= st;
+  k.up |= c & ~(c << 1);
+  if (diag) {
+    k.ul |= st & (u << 1) & ~u;
+    k.ur |= m & ~(m >> 1) & (u >> 1) & ~u;
+  }
+}
+
+// Any classes: the rows are classified once more, pixel values in hand.  Touching equal pixels
+// are joined where either run starts, or where the overlap does; diagonals as above.
+template <int CONN, class Cls>
+__device__ __forceinline__ RowMasks any_masks(const Cls& cls, const TileAt& T, int rows_in, int gx, int lane) {
+  RowMasks k = {0u, 0u, 0u, 0u, 0u};
+  unsigned same_left = 0, same_up = 0, same_ul = 0, same_ur = 0;
+  uint32_t prev = 0, prev_left = 0;
+#pragma unroll 8
+  for (int r = 0; r < kTile; ++r) {
+    const uint32_t v = (r < rows_in && gx < T.m.W) ? (uint32_t)cls(T.m, T.y0 + r, gx) : 0u;
+    const uint32_t left = __shfl_up_sync(NSGB_FULL, v, 1);
+    const bool fg = v != 0u;
+    const unsigned f = __ballot_sync(NSGB_FULL, fg);
+    const unsigned sl = __ballot_sync(NSGB_FULL, fg && lane > 0 && left == v);
+    const unsigned su = __ballot_sync(NSGB_FULL, fg && prev == v);  // prev is 0 for the first row
+    unsigned sul = 0, sur = 0;
+    if constexpr (CONN != 4) {
+      const uint32_t prev_right = __shfl_down_sync(NSGB_FULL, prev, 1);
+      const bool d = fg && joins_diagonally<CONN>(v);
+      sul = __ballot_sync(NSGB_FULL, d && lane > 0 && prev_left == v);
+      sur = __ballot_sync(NSGB_FULL, d && lane < 31 && prev_right == v);
+    }
+    if (lane == r) {
+      k.fg = f;
+      same_left = sl;
+      same_up = su;
+      same_ul = sul;
+      same_ur = sur;
+    }
+    prev = v;
+    prev_left = left;
+  }
+  k.start = k.fg & ~same_left;
+  const unsigned start_above = above(k.start, lane);
+  k.up = same_up & (~(same_up << 1) | k.start | start_above);
+  k.ul = same_ul & k.start & ~same_up;
+  k.ur = same_ur & ~(same_left >> 1) & ~same_up;
+  return k;
+}
+
+// Column of the start at or before column x.
+__device__ __forceinline__ int start_at(unsigned starts, int x) { return 31 - __clz(starts & (0xFFFFFFFFu >> (31 - x))); }
+
+// Tile-local labelling: one warp per 32 x 32 tile.  The pixels of a row become bit masks (ballots
+// over lane = column; lane r keeps row r), and from there on lane = row works on whole runs with
+// bit operations.  Runs of equal class along a row start out joined (node = run start).  A pair of
+// touching runs of adjacent rows is one contact:
+//   - each run's first contact is a plain store (its parent is the run above; parents are smaller,
+//     so this is a forest), and pointer jumping in lockstep flattens it in at most five rounds --
+//     for blobs that is nearly all there is;
+//   - the remaining contacts (a run that touches two runs above) are unions in shared memory.
+// Each run then adds its length to its root's area and puts its label at its start, and the
+// labels are written lane = column, every pixel through the start of its run.
+//
+// Bound: instructions issued (63% of cycles).  The kernel it replaced (a 256-thread CTA per tile,
+// unions, finds and area counts per pixel) issued about 5200 warp instructions per mixed tile,
+// this one 1200 (one class) to 1450 (two).  4096^2 u8, cold: two classes with areas 102 -> 38 us,
+// a 0 / 255 mask 76 -> 32 us; from a bit plane, 71 Mpixel of uneven tiles: 109 -> 49 us.
 template <class Cls, int CONN>
-__global__ void __launch_bounds__(kThreads) ccl_local(Cls cls, Imgs I, Forest f) {
+__global__ void __launch_bounds__(32 * kLocalWarps) ccl_local(Cls cls, Imgs I, Forest f, int ntiles) {
   pdl_wait();
   pdl_release();
-  using CT = typename class_type<Cls>::type;
-  __shared__ int s_lab[kTile * kTile];
-  __shared__ int s_cnt[kTile * kTile];
-  __shared__ CT s_c[kTile * kTile];
-  __shared__ CT s_wv[kThreads / 32];  // per warp: the class of its first pixel
-  const TileAt T = tile_at(I, blockIdx.x);
-  const int x0 = T.x0, y0 = T.y0, H = T.m.H, W = T.m.W, pb = T.m.px_base;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  CT c[kRows];
-#pragma unroll
-  for (int k = 0; k < kRows; ++k) {
-    const int ly = kRows * ty + k, i = ly * kTile + tx;
-    const int gy = y0 + ly, gx = x0 + tx;
-    c[k] = (CT)((gy < H && gx < W) ? cls(T.m, gy, gx) : 0u);
-    s_c[i] = c[k];
-    if (f.A) s_cnt[i] = 0;
-  }
-  // Uniform warp (one class in all its rows): one run per row, or none; no ballots needed.
-  const CT ref = (CT)__shfl_sync(NSGB_FULL, (uint32_t)c[0], 0);
-  bool same = true;
-#pragma unroll
-  for (int k = 0; k < kRows; ++k) same = same && c[k] == ref;
-  const bool wu = __all_sync(NSGB_FULL, same);
-  if (tx == 0) s_wv[ty] = ref;
-  unsigned same_left[kRows];
-  if (wu) {
-#pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      const int ly = kRows * ty + k;
-      same_left[k] = ref ? 0xFFFFFFFEu : 0u;
-      s_lab[ly * kTile + tx] = ref ? ly * kTile : -1;
-    }
+  __shared__ int s_nodes[kLocalWarps][kTile * kTile];
+  __shared__ unsigned s_starts[kLocalWarps][kTile];
+  const int b = blockIdx.x * kLocalWarps + (threadIdx.x >> 5);
+  if (b >= ntiles) return;  // whole warp; the warps of a CTA are independent
+  int* s = s_nodes[threadIdx.x >> 5];
+  unsigned* starts = s_starts[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const TileAt T = tile_at(I, b);
+  const int x0 = T.x0, y0 = T.y0, W = T.m.W, pb = T.m.px_base;
+  const int gx = x0 + lane;
+  const unsigned cols_in = W - x0 >= 32 ? 0xFFFFFFFFu : (1u << (W - x0)) - 1u;
+  const int rows_in = min(kTile, T.m.H - y0);
+
+  // (1) lane r: the masks of row r
+  RowMasks k = {0u, 0u, 0u, 0u, 0u};
+  if constexpr (Cls::kKind == kRowBits) {
+    const unsigned m = lane < rows_in ? cls.row_bits(T.m, y0 + lane, x0) & cols_in : 0u;
+    class_masks(m, joins_diagonally<CONN>(1u), lane, k);
+  } else if constexpr (Cls::kKind == kAnyClass && sizeof(typename class_type<Cls>::type) > 1) {
+    k = any_masks<CONN>(cls, T, rows_in, gx, lane);
   } else {
+    unsigned m = 0;
+    uint32_t any = 0u, all = ~0u;  // of the non-zero values (kAnyClass)
+    // Past the image edge the last row or column is read again and masked off below: loads
+    // without a predicate all go out before the first ballot (guarded ones came one by one:
+    // 71 against 30 us for the two classes of a 4096^2 u8 tile).
+    const int cx = min(gx, W - 1);
 #pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      const int ly = kRows * ty + k, i = ly * kTile + tx;
-      const CT left = (CT)__shfl_up_sync(NSGB_FULL, (uint32_t)c[k], 1);
-      same_left[k] = __ballot_sync(NSGB_FULL, tx > 0 && c[k] != 0 && left == c[k]);
-      // run start: highest lane <= tx whose pixel does not continue a run from the left
-      const unsigned starts = ~same_left[k] & (0xFFFFFFFFu >> (31 - tx));
-      const int rs = 31 - __clz(starts);
-      s_lab[i] = c[k] ? ly * kTile + rs : -1;
-    }
-  }
-  const bool all_wu = __syncthreads_and(wu) != 0;
-  // Uniform tile (one class everywhere, pixels outside the image counting as background): the
-  // whole tile is one component rooted at its first pixel, or background.  Common in masks
-  // (empty background, solid foreground), and it needs no unions.
-  if (all_wu) {
-    bool uni = true;
-#pragma unroll
-    for (int w = 1; w < kThreads / 32; ++w) uni = uni && s_wv[w] == s_wv[0];
-    if (uni) {
-      const bool fg = s_wv[0] != 0;
-      const int g0 = pb + y0 * W + x0;
-#pragma unroll
-      for (int k = 0; k < kRows; ++k) {
-        const int gy = y0 + kRows * ty + k, gx = x0 + tx;
-        if (gy < H && gx < W) f.L[pb + gy * W + gx] = fg ? g0 : -1;
+    for (int r = 0; r < kTile; ++r) {
+      const uint32_t v = (uint32_t)cls(T.m, y0 + min(r, rows_in - 1), cx);
+      if constexpr (Cls::kKind == kAnyClass) {
+        any |= v;
+        all &= v ? v : ~0u;
       }
-      if (fg && threadIdx.x == 0) {
-        f.roots[atomicAdd(f.nroots, 1)] = g0;
-        if (f.A) f.A[g0] = kTile * kTile;
+      const unsigned w = __ballot_sync(NSGB_FULL, Cls::kKind == kTwoClasses ? v == 1u : v != 0u);
+      if (lane == r) m = w;
+    }
+    m = lane < rows_in ? m & cols_in : 0u;
+    // one non-zero class in the whole tile (a 0 / 255 mask), or several
+    if (Cls::kKind == kAnyClass &&
+        (__reduce_or_sync(NSGB_FULL, any) & ~__reduce_and_sync(NSGB_FULL, all)) != 0u) {
+      k = any_masks<CONN>(cls, T, rows_in, gx, lane);
+    } else {
+      class_masks(m, joins_diagonally<CONN>(1u), lane, k);
+      if constexpr (Cls::kKind == kTwoClasses)
+        class_masks(lane < rows_in ? cols_in & ~m : 0u, joins_diagonally<CONN>(2u), lane, k);
+    }
+  }
+
+  int* Lt = f.L + pb + (int64_t)y0 * W + gx;  // this lane's column of the tile
+  // (2) a tile without foreground, or one solid class: no unions
+  const bool empty = __all_sync(NSGB_FULL, k.fg == 0u);
+  const bool solid = __all_sync(NSGB_FULL, k.fg == 0xFFFFFFFFu && k.start == 1u && (lane == 0 || k.up == 1u));
+  if (empty || solid) {
+    const int g0 = pb + y0 * W + x0;
+    const int v = solid ? g0 : -1;
+    if (gx < W) {
+#pragma unroll 8
+      for (int r = 0; r < rows_in; ++r, Lt += W) *Lt = v;
+    }
+    if (solid && lane == 0) {
+      f.roots[atomicAdd(f.nroots, 1)] = g0;
+      if (f.A) f.A[g0] = kTile * kTile;
+    }
+    return;
+  }
+
+  // (3) contacts, lane = row
+  const int row = kTile * lane;
+  const unsigned start_above = above(k.start, lane);
+  unsigned up = k.up, ul = k.ul, ur = k.ur;
+  for (unsigned w = k.start; w; w &= w - 1u) {
+    const int x = __ffs(w) - 1;
+    const unsigned next = (k.start | ~k.fg) & ~(0xFFFFFFFFu >> (31 - x));  // first column past the run
+    const unsigned run = (next ? (next & (0u - next)) - 1u : 0xFFFFFFFFu) & (0xFFFFFFFFu << x);
+    int c = -1;  // the column above of the run's first contact
+    unsigned t;
+    if ((ul >> x) & 1u) {
+      ul &= ~(1u << x);
+      c = x - 1;
+    } else if ((t = up & run) != 0u) {
+      up &= ~(t & (0u - t));
+      c = __ffs(t) - 1;
+    } else if ((t = ur & run) != 0u) {
+      ur &= ~t;
+      c = __ffs(t);
+    }
+    s[node_at(row + x)] = c >= 0 ? row - kTile + start_at(start_above, c) : row + x;
+  }
+  __syncwarp();
+  for (;;) {
+    bool moved = false;
+    for (unsigned w = k.start; w; w &= w - 1u) {
+      volatile int* v = s;
+      const int i = node_at(row + __ffs(w) - 1);
+      const int p = v[i], g = v[node_at(p)];
+      if (g != p) {
+        v[i] = g;
+        moved = true;
       }
-      return;
+    }
+    if (!__any_sync(NSGB_FULL, moved)) break;
+  }
+  if (__any_sync(NSGB_FULL, (up | ul | ur) != 0u)) {
+    int d = 0;
+    for (;;) {
+      if (up == 0u) {
+        if (ul) {
+          up = ul, ul = 0u, d = -1;
+        } else if (ur) {
+          up = ur, ur = 0u, d = 1;
+        } else {
+          break;
+        }
+      }
+      const int x = __ffs(up) - 1;
+      up &= up - 1u;
+      s_union(s, row + start_at(k.start, x), row - kTile + start_at(start_above, x + d));
+    }
+    __syncwarp();
+  }
+
+  // (4) every run points at its root; run lengths add up at the roots (above bit 16)
+  unsigned is_root = 0u;
+  for (unsigned w = k.start; w; w &= w - 1u) {
+    const int x = __ffs(w) - 1, i = row + x;
+    const int r = s_find<true>(s, i);
+    if (r == i) is_root |= 1u << x;
+    else atomicMin(&s[node_at(i)], r);
+    if (f.A) {
+      const unsigned stop = (k.start | ~k.fg) & ~(0xFFFFFFFFu >> (31 - x));
+      atomicAdd(&s[node_at(r)], ((stop ? __ffs(stop) - 1 : 32) - x) << 16);
     }
   }
+  __syncwarp();
+
+  // (5) the tile's local roots go to the list with one atomic, and every run start (background
+  // runs included) gets the label of its pixels.  A lane touches only the nodes of its own row.
+  const int nr = __popc(is_root);
+  int incl = nr;
 #pragma unroll
-  for (int k = 0; k < kRows; ++k) {
-    const int ly = kRows * ty + k, i = ly * kTile + tx;
-    const CT v = c[k];
-    if (!v || ly == 0) continue;
-    const bool run_start = !((same_left[k] >> tx) & 1u);
-    const int u = i - kTile;
-    const CT up = s_c[u];
-    const bool up_start = up != 0 && !(tx > 0 && s_c[u - 1] == up);
-    if (up == v && (run_start || up_start)) s_union(s_lab, i, u);
-    if (joins_diagonally<CONN>(v)) {
-      if (run_start && tx > 0 && s_c[u - 1] == v) s_union(s_lab, i, u - 1);
-      const bool run_end = (tx == kTile - 1) || s_c[i + 1] != v;
-      if (run_end && tx < kTile - 1 && s_c[u + 1] == v) s_union(s_lab, i, u + 1);
-    }
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(NSGB_FULL, incl, o);
+    if (lane >= o) incl += v;
   }
-  __syncthreads();
-  int root[kRows];
-#pragma unroll
-  for (int k = 0; k < kRows; ++k) {
-    const int ly = kRows * ty + k, i = ly * kTile + tx;
-    root[k] = c[k] ? s_find(s_lab, i) : -1;
-  }
-  if (f.A) {
-#pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      const int r = root[k];
-      const unsigned peers = __match_any_sync(NSGB_FULL, r);
-      if (r >= 0 && (__ffs(peers) - 1) == tx) atomicAdd(&s_cnt[r], __popc(peers));
-    }
-    __syncthreads();
-  }
-  unsigned rb[kRows];
-  int nr = 0;
-#pragma unroll
-  for (int k = 0; k < kRows; ++k) {
-    const int ly = kRows * ty + k, i = ly * kTile + tx;
-    const int gy = y0 + ly, gx = x0 + tx;
-    const bool in = gy < H && gx < W;
-    const int r = root[k];
-    const int g = pb + gy * W + gx;
-    if (in) f.L[g] = r < 0 ? -1 : pb + (y0 + r / kTile) * W + x0 + (r % kTile);
-    rb[k] = __ballot_sync(NSGB_FULL, in && r == i);
-    nr += __popc(rb[k]);
-  }
-  // The warp's local roots (all four rows) go to the list with one atomic: a tile of singleton
-  // components has 1024 roots, and per-row atomics on the one counter would serialise.
-  if (nr == 0) return;  // warp-uniform: most warps of a labelling hold no root
   int base = 0;
-  if (tx == 0) base = atomicAdd(f.nroots, nr);
-  base = __shfl_sync(NSGB_FULL, base, 0);
-#pragma unroll
-  for (int k = 0; k < kRows; ++k) {
-    if ((rb[k] >> tx) & 1u) {
-      const int ly = kRows * ty + k, i = ly * kTile + tx;
-      const int g = pb + (y0 + ly) * W + x0 + tx;
-      f.roots[base + __popc(rb[k] & ((1u << tx) - 1u))] = g;
-      if (f.A) f.A[g] = s_cnt[i];
+  if (lane == 31) base = atomicAdd(f.nroots, incl);
+  base = __shfl_sync(NSGB_FULL, base, 31) + incl - nr;
+  const unsigned every = k.start | (~k.fg & ((k.fg << 1) | 1u));
+  starts[lane] = every;
+  for (unsigned w = every; w; w &= w - 1u) {
+    const int x = __ffs(w) - 1;
+    int* const node = &s[node_at(row + x)];
+    int label = -1;
+    if ((k.fg >> x) & 1u) {
+      const int v = *node, q = v & kNodeMask;
+      label = pb + (y0 + (q >> 5)) * W + x0 + (q & 31);
+      if ((is_root >> x) & 1u) {
+        f.roots[base++] = label;
+        if (f.A) f.A[label] = v >> 16;
+      }
     }
-    base += __popc(rb[k]);
+    *node = label;
+  }
+  __syncwarp();
+
+  // (6) labels, lane = column
+  if (gx < W) {
+    const unsigned upto = 0xFFFFFFFFu >> (31 - lane);
+#pragma unroll 8
+    for (int r = 0; r < rows_in; ++r, Lt += W) *Lt = s[node_at(kTile * r + 31 - __clz(starts[r] & upto))];
   }
 }
 
@@ -585,6 +717,8 @@ inline dim3 quadrow_grid(int total_rows, int max_w) {
   return dim3(bx, row_blocks(total_rows));
 }
 
+inline unsigned local_grid(int c_tiles) { return (unsigned)((c_tiles + kLocalWarps - 1) / kLocalWarps); }
+
 // Labels every image of the batch: local pass, edge merge, root flattening.  Afterwards
 // root(i) = L[L[i]].
 template <class Cls>
@@ -592,10 +726,10 @@ cudaError_t label(const Cls& cls, const Imgs& I, const BatchTotals& t, int conn,
   cudaError_t e = cudaMemsetAsync(f.nroots, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
   if (conn == 8) {
-    ccl_local<Cls, 8><<<t.c_tiles, kThreads, 0, s>>>(cls, I, f);
+    ccl_local<Cls, 8><<<local_grid(t.c_tiles), 32 * kLocalWarps, 0, s>>>(cls, I, f, t.c_tiles);
     ccl_merge<Cls, 8><<<t.c_tiles, 64, 0, s>>>(cls, I, f.L);
   } else {
-    ccl_local<Cls, 4><<<t.c_tiles, kThreads, 0, s>>>(cls, I, f);
+    ccl_local<Cls, 4><<<local_grid(t.c_tiles), 32 * kLocalWarps, 0, s>>>(cls, I, f, t.c_tiles);
     ccl_merge<Cls, 4><<<t.c_tiles, 64, 0, s>>>(cls, I, f.L);
   }
   ccl_flatten_roots<<<list_grid(t.px), 256, 0, s>>>(f, (int)t.px);
@@ -683,10 +817,10 @@ cudaError_t label_filled(const Cls& cls, const Imgs& I, const BatchTotals& t, in
   cudaError_t e = launch_k(false, zero_words, dim3(flat_grid(z.total())), dim3(256), s, z);
   if (e != cudaSuccess) return e;
   if (conn == kConnFg8Bg4) {
-    e = launch_k(pdl, ccl_local<Cls, kConnFg8Bg4>, dim3(t.c_tiles), dim3(kThreads), s, cls, I, f);
+    e = launch_k(pdl, ccl_local<Cls, kConnFg8Bg4>, dim3(local_grid(t.c_tiles)), dim3(32 * kLocalWarps), s, cls, I, f, t.c_tiles);
     if (e == cudaSuccess) e = launch_k(pdl, ccl_merge<Cls, kConnFg8Bg4>, dim3(t.c_tiles), dim3(64), s, cls, I, f.L);
   } else {
-    e = launch_k(pdl, ccl_local<Cls, kConnFg4Bg8>, dim3(t.c_tiles), dim3(kThreads), s, cls, I, f);
+    e = launch_k(pdl, ccl_local<Cls, kConnFg4Bg8>, dim3(local_grid(t.c_tiles)), dim3(32 * kLocalWarps), s, cls, I, f, t.c_tiles);
     if (e == cudaSuccess) e = launch_k(pdl, ccl_merge<Cls, kConnFg4Bg8>, dim3(t.c_tiles), dim3(64), s, cls, I, f.L);
   }
   const int gx = (t.perimeter_max + 255) / 256 > 64 ? 64 : (t.perimeter_max + 255) / 256;

@@ -37,6 +37,12 @@ template <typename T>
 __device__ __forceinline__ T pxcg(const void* base, int64_t pitch, int y, int x) {
   return __ldcg((const T*)((const char*)base + (int64_t)y * pitch) + x);
 }
+// A plain load, for planes an earlier launch wrote: unlike the one above it can be batched with
+// its neighbours by the compiler (32 rows of a labelling tile in flight at once).
+template <typename T>
+__device__ __forceinline__ T pxw(const void* base, int64_t pitch, int y, int x) {
+  return *((const T*)((const char*)base + (int64_t)y * pitch) + x);
+}
 template <typename T>
 __device__ __forceinline__ T* pxp(void* base, int64_t pitch, int y, int x) {
   return (T*)((char*)base + (int64_t)y * pitch) + x;
@@ -49,23 +55,24 @@ __device__ __forceinline__ T* pxp(void* base, int64_t pitch, int y, int x) {
 // OpenCV's compare converts the scalar to the image's depth.  Both are prepared on the host.
 template <typename T>
 struct GtThr {
-  using K = std::conditional_t<std::is_floating_point<T>::value, float, int64_t>;
-  K k;
+  using K = std::conditional_t<std::is_floating_point<T>::value, float, int>;
+  K k;        // integers: the smallest value above the threshold
+  bool none;  // integers: nothing is above it
   static GtThr make(double thr) {
     GtThr g;
+    g.none = false;
     if constexpr (std::is_floating_point<T>::value) {
       g.k = (float)thr;
     } else {
-      if (thr != thr) g.k = INT64_MAX;  // NaN: nothing is greater
-      else if (thr >= 9.0e18) g.k = INT64_MAX;
-      else if (thr <= -9.0e18) g.k = INT64_MIN;
-      else g.k = (int64_t)floor(thr);
+      const double f = floor(thr);
+      g.none = !(f < (double)INT_MAX);  // NaN: nothing is greater
+      g.k = g.none ? INT_MAX : f < (double)INT_MIN ? INT_MIN : (int)f + 1;
     }
     return g;
   }
   __device__ __forceinline__ bool operator()(T x) const {
     if constexpr (std::is_floating_point<T>::value) return x > k;
-    else return (int64_t)x > k;
+    else return (int)x >= k && !none;
   }
 };
 
@@ -73,23 +80,31 @@ struct GtThr {
 // Classifiers (class 0 = background; equal non-zero classes are joined).  They read the
 // image's plane (Img::plane) or aux plane.
 struct ClsValueU8 {  // bwlabel: the pixel value
+  static constexpr ccl::ClassKind kKind = ccl::kAnyClass;
   __device__ uint32_t operator()(const Img& m, int y, int x) const { return px<uint8_t>(m.plane, m.pitch, y, x); }
 };
 struct ClsNotFlooded {  // a batch's filled image: the pixels the flood from outside did not reach
+  static constexpr ccl::ClassKind kKind = ccl::kRowBits;
   const uint32_t* flooded;  // bit plane, rows of bit_words(W) words from Img::b_base
   __device__ uint32_t operator()(const Img& m, int y, int x) const {
     const uint32_t w = __ldg(flooded + m.b_base + (int64_t)y * ((m.W + 31) / 32) + (x >> 5));
     return ((w >> (x & 31)) & 1u) ^ 1u;
   }
+  // columns x .. x + 31 of row y (x a multiple of 32)
+  __device__ uint32_t row_bits(const Img& m, int y, int x) const {
+    return ~__ldg(flooded + m.b_base + (int64_t)y * ((m.W + 31) / 32) + (x >> 5));
+  }
 };
 struct ClsDenseU8 {  // the chain's filled image F in the workspace (dense, at px_base)
+  static constexpr ccl::ClassKind kKind = ccl::kOneClass;
   const uint8_t* F;
   __device__ uint32_t operator()(const Img& m, int y, int x) const {
-    return __ldg(F + m.px_base + (int64_t)y * m.W + x);
+    return __ldg(F + m.px_base + (int64_t)y * m.W + x) != 0 ? 1u : 0u;
   }
 };
 template <typename T>
 struct ClsNonZero {  // binary reconstruction (mask = aux), bwselect (image = plane)
+  static constexpr ccl::ClassKind kKind = ccl::kOneClass;
   bool use_aux;
   __device__ uint32_t operator()(const Img& m, int y, int x) const {
     return px<T>(use_aux ? m.aux : m.plane, m.pitch, y, x) != (T)0 ? 1u : 0u;
@@ -97,22 +112,25 @@ struct ClsNonZero {  // binary reconstruction (mask = aux), bwselect (image = pl
 };
 template <typename T>
 struct ClsNotMax {  // binary hole filling: pixels that are not foreground (max<T>)
+  static constexpr ccl::ClassKind kKind = ccl::kOneClass;
   __device__ uint32_t operator()(const Img& m, int y, int x) const {
     return px<T>(m.plane, m.pitch, y, x) != std::numeric_limits<T>::max() ? 1u : 0u;
   }
 };
 template <typename T>
 struct ClsAboveOrNot {  // hole filling and labelling at once: 1 where R > thr, 2 elsewhere
+  static constexpr ccl::ClassKind kKind = ccl::kTwoClasses;
   GtThr<T> gt;
   __device__ uint32_t operator()(const Img& m, int y, int x) const {
-    return gt(pxcg<T>(m.plane, m.pitch, y, x)) ? 1u : 2u;
+    return gt(pxw<T>(m.plane, m.pitch, y, x)) ? 1u : 2u;
   }
 };
 template <typename T>
 struct ClsNotAbove {  // hole filling of (R > thr): the complement class !(R > thr); R = plane
+  static constexpr ccl::ClassKind kKind = ccl::kOneClass;
   GtThr<T> gt;
   __device__ uint32_t operator()(const Img& m, int y, int x) const {
-    return gt(pxcg<T>(m.plane, m.pitch, y, x)) ? 0u : 1u;
+    return gt(pxw<T>(m.plane, m.pitch, y, x)) ? 0u : 1u;
   }
 };
 
@@ -120,14 +138,16 @@ struct ClsNotAbove {  // hole filling of (R > thr): the complement class !(R > t
 // Mat subtraction, HistologicalEntities.cpp:199), from the reconstruction R (plane, written by
 // an earlier launch) and the image rc it was taken under (aux).
 __device__ __forceinline__ uint8_t valley(const Img& m, int y, int x) {
-  const int d = (int)px<uint8_t>(m.aux, m.pitch, y, x) - (int)pxcg<uint8_t>(m.plane, m.pitch, y, x);
+  const int d = (int)px<uint8_t>(m.aux, m.pitch, y, x) - (int)pxw<uint8_t>(m.plane, m.pitch, y, x);
   return (uint8_t)(d > 0 ? d : 0);
 }
 struct ClsValleyAboveOrNot {  // hole filling and labelling of (D > g1) at once: 1 where D > g1, 2 elsewhere
+  static constexpr ccl::ClassKind kKind = ccl::kTwoClasses;
   GtThr<uint8_t> gt;
   __device__ uint32_t operator()(const Img& m, int y, int x) const { return gt(valley(m, y, x)) ? 1u : 2u; }
 };
 struct ClsValleyAbove {  // bwselect's image D > g2
+  static constexpr ccl::ClassKind kKind = ccl::kOneClass;
   GtThr<uint8_t> gt;
   __device__ uint32_t operator()(const Img& m, int y, int x) const { return gt(valley(m, y, x)) ? 1u : 0u; }
 };
@@ -1457,6 +1477,7 @@ constexpr int kKeyNone = 0x7F7F7F7F;  // memset byte 0x7F: no source seen yet
 
 // Plateau class: all 32 bits of R (+0 and -0 merged), plus one so that no value is background.
 struct ClsPlateau {
+  static constexpr ccl::ClassKind kKind = ccl::kAnyClass;
   using class_t = uint32_t;
   __device__ uint32_t operator()(const Img& m, int y, int x) const {
     uint32_t v = __float_as_uint(pxcg<float>(m.plane, m.pitch, y, x));
