@@ -13,13 +13,17 @@ constexpr int kMorphMaxK = 63;  // largest structuring element side (half-width 
 // A k x k structuring element (k odd), as the kernels read it.  Row `i` of the element is the
 // image row offset i - bw; `row_bits[i]` bit j = element (i, j) non-zero, column offset j - bw.
 // `radius[i]` >= 0 when row i is one run of columns centred on the middle column (bw - r ..
-// bw + r), -1 when it is empty; `dy_of_radius[r]` = the rows whose run has radius r.  `centred`:
-// every non-empty row is such a run (disks, rectangles, diamonds), which takes the fast path.
+// bw + r), -1 when it is empty.  `centred`: every non-empty row is such a run (disks, rectangles,
+// diamonds), which takes the fast path.  The rows of radius r are then the vertical runs
+// first_run[r] .. first_run[r + 1] - 1: `run_len` consecutive element rows from `run_row`; bit r of
+// `radii` is set when there are any.
 struct MorphElement {
   int k, bw, centred, max_radius;
+  uint32_t radii;
   uint64_t row_bits[kMorphMaxK];
   int8_t radius[kMorphMaxK + 1];
-  uint64_t dy_of_radius[kMorphMaxK / 2 + 1];
+  uint8_t first_run[kMorphMaxK / 2 + 2];
+  uint8_t run_row[kMorphMaxK], run_len[kMorphMaxK];
 };
 
 // Builds the element from a host k x k array (non-zero = in the element).  Returns false for an
