@@ -102,6 +102,7 @@ struct Px<uint8_t> {
   static constexpr uint32_t LOW = 0u, HIGH = 0xFFFFFFFFu, FLIP = 0x00FF00FFu, ZERO = 0u;
   static constexpr uint32_t ELEM_FLIP = 0xFFu;
   __device__ static __forceinline__ uint32_t vmax(uint32_t a, uint32_t b) { return vmax_u16x2(a, b); }
+  __device__ static __forceinline__ uint32_t vmax3(uint32_t a, uint32_t b, uint32_t c) { return __vimax3_u16x2(a, b, c); }
   __device__ static __forceinline__ uint32_t vmin(uint32_t a, uint32_t b) { return vmin_u16x2(a, b); }
   // element k <- element k-1, element 0 <- last element of prev
   __device__ static __forceinline__ uint32_t from_left(uint32_t prev, uint32_t cur) { return __funnelshift_l(prev, cur, 16); }
@@ -126,6 +127,7 @@ struct Px<uint16_t> {
   static constexpr uint32_t LOW = 0u, HIGH = 0xFFFFFFFFu, FLIP = 0xFFFFFFFFu, ZERO = 0u;
   static constexpr uint32_t ELEM_FLIP = 0xFFFFu;
   __device__ static __forceinline__ uint32_t vmax(uint32_t a, uint32_t b) { return vmax_u16x2(a, b); }
+  __device__ static __forceinline__ uint32_t vmax3(uint32_t a, uint32_t b, uint32_t c) { return __vimax3_u16x2(a, b, c); }
   __device__ static __forceinline__ uint32_t vmin(uint32_t a, uint32_t b) { return vmin_u16x2(a, b); }
   __device__ static __forceinline__ uint32_t from_left(uint32_t prev, uint32_t cur) { return __funnelshift_l(prev, cur, 16); }
   __device__ static __forceinline__ uint32_t from_right(uint32_t cur, uint32_t next) { return __funnelshift_r(cur, next, 16); }
@@ -147,6 +149,9 @@ struct Px<int32_t> {
   static constexpr uint32_t LOW = 0x80000000u, HIGH = 0x7FFFFFFFu, FLIP = 0xFFFFFFFFu, ZERO = 0u;
   static constexpr uint32_t ELEM_FLIP = 0xFFFFFFFFu;
   __device__ static __forceinline__ uint32_t vmax(uint32_t a, uint32_t b) { return (uint32_t)max((int)a, (int)b); }
+  __device__ static __forceinline__ uint32_t vmax3(uint32_t a, uint32_t b, uint32_t c) {
+    return (uint32_t)__vimax3_s32((int)a, (int)b, (int)c);
+  }
   __device__ static __forceinline__ uint32_t vmin(uint32_t a, uint32_t b) { return (uint32_t)min((int)a, (int)b); }
   __device__ static __forceinline__ uint32_t from_left(uint32_t prev, uint32_t) { return prev; }
   __device__ static __forceinline__ uint32_t from_right(uint32_t, uint32_t next) { return next; }
@@ -169,6 +174,11 @@ struct Px<float> {
   static constexpr uint32_t ELEM_FLIP = 0x80000000u;
   __device__ static __forceinline__ uint32_t vmax(uint32_t a, uint32_t b) {
     return __float_as_uint(fmaxf(__uint_as_float(a), __uint_as_float(b)));
+  }
+  __device__ static __forceinline__ uint32_t vmax3(uint32_t a, uint32_t b, uint32_t c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(__uint_as_float(a)), "f"(__uint_as_float(b)), "f"(__uint_as_float(c)));
+    return __float_as_uint(r);
   }
   __device__ static __forceinline__ uint32_t vmin(uint32_t a, uint32_t b) {
     return __float_as_uint(fminf(__uint_as_float(a), __uint_as_float(b)));

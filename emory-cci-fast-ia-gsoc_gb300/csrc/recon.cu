@@ -108,18 +108,22 @@ __device__ __forceinline__ T* row_ptr(T* base, int64_t pitch, int y) {
   return (T*)((char*)base + (int64_t)y * pitch);
 }
 
+__device__ __forceinline__ int clamped(int v, int n) { return min(max(v, 0), n - 1); }
+
 // Loads the word holding elements (y, x .. x+E-1), flipped into the working order; elements
-// outside the image read as LOW.  `coherent` selects L2-coherent loads for planes that other
+// outside the image read as LOW.  Outside, the nearest pixel is loaded and dropped: a load behind
+// a test of its coordinates waits for the one before it, and the halo of a tile is 16 loads (a
+// tile's loads took 17900 cycles of a 32-bit visit, most of them one halo load after another).  `coherent` selects L2-coherent loads for planes that other
 // warps write during the kernel.
 template <typename T>
 __device__ __forceinline__ uint32_t load_word(const T* base, int64_t pitch, int y, int x, int H, int W,
                                               bool fast, bool coherent, bool flip) {
   using P = Px<T>;
   const uint32_t ef = flip ? P::ELEM_FLIP : 0u;
-  if (y < 0 || y >= H) return P::LOW;
-  const T* r = row_ptr(base, pitch, y) + x;
+  const int yc = clamped(y, H);
   if constexpr (P::E == 2) {
-    if (fast) {
+    if (fast) {  // the row is inside
+      const T* r = row_ptr(base, pitch, y) + x;
       uint32_t w;
       if constexpr (sizeof(T) == 1) {
         unsigned short v = coherent ? __ldcg((const unsigned short*)r) : __ldg((const unsigned short*)r);
@@ -129,13 +133,15 @@ __device__ __forceinline__ uint32_t load_word(const T* base, int64_t pitch, int 
       }
       return w ^ (flip ? P::FLIP : 0u);
     }
-    uint32_t e0 = P::LOW, e1 = P::LOW;
-    if (x >= 0 && x < W) e0 = (coherent ? P::load_elem(r) : P::load_elem_ro(r)) ^ ef;
-    if (x + 1 >= 0 && x + 1 < W) e1 = (coherent ? P::load_elem(r + 1) : P::load_elem_ro(r + 1)) ^ ef;
-    return P::pack(e0, e1);
+    const T *p0 = row_ptr(base, pitch, yc) + clamped(x, W), *p1 = row_ptr(base, pitch, yc) + clamped(x + 1, W);
+    const uint32_t v0 = coherent ? P::load_elem(p0) : P::load_elem_ro(p0);
+    const uint32_t v1 = coherent ? P::load_elem(p1) : P::load_elem_ro(p1);
+    return P::pack(yc == y && (unsigned)x < (unsigned)W ? v0 ^ ef : P::LOW,
+                   yc == y && (unsigned)(x + 1) < (unsigned)W ? v1 ^ ef : P::LOW);
   } else {
-    if (x < 0 || x >= W) return P::LOW;
-    return (coherent ? P::load_elem(r) : P::load_elem_ro(r)) ^ ef;
+    const T* p = row_ptr(base, pitch, yc) + clamped(x, W);
+    const uint32_t v = coherent ? P::load_elem(p) : P::load_elem_ro(p);
+    return yc == y && (unsigned)x < (unsigned)W ? v ^ ef : P::LOW;
   }
 }
 
@@ -163,30 +169,37 @@ __device__ __forceinline__ void store_word(T* base, int64_t pitch, int y, int x,
   }
 }
 
-// Interior-tile word access at a precomputed address (flip = xor with fx).
+// Interior-tile word access at a precomputed address: fast_load() gives the word as loaded,
+// fast_word() the compute word (flip = xor with fx).  Loading and converting are separate so that
+// every load of a tile goes out before the first conversion waits for one (a warp barrier between
+// the two keeps the compiler from mixing them).
 // `pairs`: the two elements of a 16-bit-lane word are loaded (stored) separately, for images
 // whose rows are not word aligned (an odd u8 width, say); the choice is the same for the whole
 // image, so it never diverges.
 template <typename T>
-__device__ __forceinline__ uint32_t fast_word(const char* p, bool coherent, uint32_t fx, bool pairs) {
+__device__ __forceinline__ uint32_t fast_load(const char* p, bool coherent, bool pairs) {
   if constexpr (sizeof(T) == 1) {
     if (pairs) {
       const uint32_t b0 = coherent ? __ldcg((const unsigned char*)p) : __ldg((const unsigned char*)p);
       const uint32_t b1 = coherent ? __ldcg((const unsigned char*)p + 1) : __ldg((const unsigned char*)p + 1);
-      return (b0 | (b1 << 16)) ^ fx;
+      return b0 | (b1 << 16);
     }
-    const unsigned short v = coherent ? __ldcg((const unsigned short*)p) : __ldg((const unsigned short*)p);
-    return __byte_perm((uint32_t)v, 0u, 0x7170) ^ fx;  // bytes b0,b1 -> 16-bit lanes
+    return coherent ? __ldcg((const unsigned short*)p) : __ldg((const unsigned short*)p);
   } else if constexpr (sizeof(T) == 2) {
     if (pairs) {
       const uint32_t h0 = coherent ? __ldcg((const unsigned short*)p) : __ldg((const unsigned short*)p);
       const uint32_t h1 = coherent ? __ldcg((const unsigned short*)p + 1) : __ldg((const unsigned short*)p + 1);
-      return (h0 | (h1 << 16)) ^ fx;
+      return h0 | (h1 << 16);
     }
-    return (coherent ? __ldcg((const unsigned int*)p) : __ldg((const unsigned int*)p)) ^ fx;
+    return coherent ? __ldcg((const unsigned int*)p) : __ldg((const unsigned int*)p);
   } else {
-    return (coherent ? __ldcg((const unsigned int*)p) : __ldg((const unsigned int*)p)) ^ fx;
+    return coherent ? __ldcg((const unsigned int*)p) : __ldg((const unsigned int*)p);
   }
+}
+template <typename T>
+__device__ __forceinline__ uint32_t fast_word(uint32_t raw, uint32_t fx, bool pairs) {
+  if (sizeof(T) == 1 && !pairs) raw = __byte_perm(raw, 0u, 0x7170);  // bytes b0,b1 -> 16-bit lanes
+  return raw ^ fx;
 }
 
 template <typename T>
@@ -233,9 +246,10 @@ template <typename T>
 __device__ __forceinline__ uint32_t load_elem_at(const T* base, int64_t pitch, int y, int x, int H, int W,
                                                  bool coherent, bool flip) {
   using P = Px<T>;
-  if (y < 0 || y >= H || x < 0 || x >= W) return P::LOW;
-  const T* r = row_ptr(base, pitch, y) + x;
-  return (coherent ? P::load_elem(r) : P::load_elem_ro(r)) ^ (flip ? P::ELEM_FLIP : 0u);
+  const int yc = clamped(y, H), xc = clamped(x, W);
+  const T* r = row_ptr(base, pitch, yc) + xc;
+  const uint32_t v = (coherent ? P::load_elem(r) : P::load_elem_ro(r)) ^ (flip ? P::ELEM_FLIP : 0u);
+  return yc == y && xc == x ? v : P::LOW;
 }
 
 __device__ __forceinline__ void sts2(uint32_t* p, uint32_t a, uint32_t b) {
@@ -398,7 +412,7 @@ __device__ __forceinline__ uint32_t col_step(uint32_t o, uint32_t prev, uint32_t
   if constexpr (CONN == 8) {
     const uint32_t l = __shfl_up_sync(NSGB_FULL, prev, 1);
     const uint32_t r = __shfl_down_sync(NSGB_FULL, prev, 1);
-    return P::vmin(P::vmax(t, P::vmax(P::from_left(l, prev), P::from_right(prev, r))), m);
+    return P::vmin(P::vmax3(t, P::from_left(l, prev), P::from_right(prev, r)), m);
   } else {
     return P::vmin(t, m);
   }
@@ -587,12 +601,12 @@ __device__ __forceinline__ void visit(const Args& a, WarpBuf& B, int t, int lane
   if (fast) {
     const char* mp = (const char*)mask + (int64_t)y0 * pitch + (int64_t)xl * sizeof(T);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) M[i] = fast_word<T>(mp + i * pitch, false, fx, pairs);
+    for (int i = 0; i < 32; ++i) M[i] = fast_load<T>(mp + i * pitch, false, pairs);
   }
   if (fast) {  // interior tile: straight-line loads through running row pointers, no checks
     const char* op = (const char*)src + (int64_t)y0 * pitch + (int64_t)xl * sizeof(T);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) O[i] = fast_word<T>(op + i * pitch, true, fx, pairs);
+    for (int i = 0; i < 32; ++i) O[i] = fast_load<T>(op + i * pitch, true, pairs);
   } else {
     // Edge tile: bounds-checked loads in a rolled loop through shared memory
     // (keeps this rarely used path out of the instruction cache's way).
@@ -620,12 +634,19 @@ __device__ __forceinline__ void visit(const Args& a, WarpBuf& B, int t, int lane
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int k = lane + 32 * j;
-    const int y = y0 - 1 + k;
-    const bool ok = k < 34;
-    hm[2 * j] = ok ? load_elem_at<T>(mask, pitch, y, x0 - 1, H, W, false, flip) : P::LOW;
-    hm[2 * j + 1] = ok ? load_elem_at<T>(mask, pitch, y, x0 + TW, H, W, false, flip) : P::LOW;
-    hv[2 * j] = ok ? load_elem_at<T>(src, pitch, y, x0 - 1, H, W, coh, flip) : P::LOW;
-    hv[2 * j + 1] = ok ? load_elem_at<T>(src, pitch, y, x0 + TW, H, W, coh, flip) : P::LOW;
+    const int y = y0 - 1 + min(k, 33);
+    hm[2 * j] = load_elem_at<T>(mask, pitch, y, x0 - 1, H, W, false, flip);
+    hm[2 * j + 1] = load_elem_at<T>(mask, pitch, y, x0 + TW, H, W, false, flip);
+    hv[2 * j] = load_elem_at<T>(src, pitch, y, x0 - 1, H, W, coh, flip);
+    hv[2 * j + 1] = load_elem_at<T>(src, pitch, y, x0 + TW, H, W, coh, flip);
+  }
+  __syncwarp();
+  if (fast) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      M[i] = fast_word<T>(M[i], fx, pairs);
+      O[i] = fast_word<T>(O[i], fx, pairs);
+    }
   }
   // any_change: did this visit change a stored value (the clamp to the mask on load counts).
   uint32_t any_change = 0;
@@ -810,10 +831,9 @@ __device__ __forceinline__ void visit(const Args& a, WarpBuf& B, int t, int lane
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int k = lane + 32 * j;
-      const int y = y0 - 1 + k;
-      const bool ok = k < 34;
-      hv[2 * j] = ok ? load_elem_at<T>(src, pitch, y, x0 - 1, H, W, coh, flip) : P::LOW;
-      hv[2 * j + 1] = ok ? load_elem_at<T>(src, pitch, y, x0 + TW, H, W, coh, flip) : P::LOW;
+      const int y = y0 - 1 + min(k, 33);
+      hv[2 * j] = load_elem_at<T>(src, pitch, y, x0 - 1, H, W, coh, flip);
+      hv[2 * j + 1] = load_elem_at<T>(src, pitch, y, x0 + TW, H, W, coh, flip);
     }
     topv = init_word<T>(tv, topm, y0 - 1, xl, H, W, ring);
     botv = init_word<T>(bv, botm, y0 + kRows, xl, H, W, ring);
@@ -887,9 +907,9 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, WarpBuf& B, int t, 
     const char* mp = (const char*)mask + (int64_t)y0 * pitch + (int64_t)xl * sizeof(T);
     const char* op = (const char*)out + (int64_t)y0 * pitch + (int64_t)xl * sizeof(T);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) M[i] = fast_word<T>(mp + i * pitch, false, fx, pairs);
+    for (int i = 0; i < 32; ++i) M[i] = fast_load<T>(mp + i * pitch, false, pairs);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) O[i] = fast_word<T>(op + i * pitch, true, fx, pairs);
+    for (int i = 0; i < 32; ++i) O[i] = fast_load<T>(op + i * pitch, true, pairs);
   } else {
 #pragma unroll 1
     for (int i = 0; i < 32; ++i) {
@@ -914,12 +934,19 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, WarpBuf& B, int t, 
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int k = lane + 32 * j;
-    const int y = y0 - 1 + k;
-    const bool ok = k < 34;
-    hm[2 * j] = ok ? load_elem_at<T>(mask, pitch, y, x0 - 1, H, W, false, flip) : P::LOW;
-    hm[2 * j + 1] = ok ? load_elem_at<T>(mask, pitch, y, x0 + TW, H, W, false, flip) : P::LOW;
-    hv[2 * j] = ok ? load_elem_at<T>(out, pitch, y, x0 - 1, H, W, true, flip) : P::LOW;
-    hv[2 * j + 1] = ok ? load_elem_at<T>(out, pitch, y, x0 + TW, H, W, true, flip) : P::LOW;
+    const int y = y0 - 1 + min(k, 33);
+    hm[2 * j] = load_elem_at<T>(mask, pitch, y, x0 - 1, H, W, false, flip);
+    hm[2 * j + 1] = load_elem_at<T>(mask, pitch, y, x0 + TW, H, W, false, flip);
+    hv[2 * j] = load_elem_at<T>(out, pitch, y, x0 - 1, H, W, true, flip);
+    hv[2 * j + 1] = load_elem_at<T>(out, pitch, y, x0 + TW, H, W, true, flip);
+  }
+  __syncwarp();
+  if (fast) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      M[i] = fast_word<T>(M[i], fx, pairs);
+      O[i] = fast_word<T>(O[i], fx, pairs);
+    }
   }
   uint32_t any_change = 0;
 #pragma unroll
