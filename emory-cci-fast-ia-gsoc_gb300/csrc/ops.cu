@@ -1576,7 +1576,7 @@ __device__ __forceinline__ bool fix_from_float(float g, Fix128& out) {
   // fixed = man * 2^(sh + 96)
   unsigned long long lo = 0, hi = 0;
   const int s = sh + 96;
-  if (s >= 0) {  // s <= 157 - 150 + 96 - 1 = 102, man < 2^24: fits in 126 bits
+  if (s >= 0) {  // s <= 157 - 150 + 96 = 103, man < 2^24: fits in 127 bits
     if (s < 64) {
       lo = (unsigned long long)man << s;
       hi = s == 0 ? 0ull : (unsigned long long)man >> (64 - s);
@@ -1648,87 +1648,402 @@ __device__ __forceinline__ float fix_to_float(unsigned long long lo, long long h
   return __uint_as_float(bits);
 }
 
-// Adjoint, pass 1: every pixel adds its gradient, as an exact 128-bit fixed-point value, to the
-// accumulator of its source.  Lanes of a warp hold consecutive pixels of one row, which mostly
-// share a source: a segmented warp scan sums runs of equal targets first, so only the last lane
-// of each run issues the atomics (low word, then the high word with the low word's carry).
-// plane = g, aux = prov.  acc: two words per source, marker sources then mask sources.
-__global__ void grad_scatter_kernel(Imgs I, int total_rows, unsigned long long* __restrict__ acc_marker,
-                                    unsigned long long* __restrict__ acc_mask, int* status) {
-  const int lane = threadIdx.x & 31;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  for (int gr = blockIdx.y; gr < total_rows; gr += gridDim.y) {  // uniform per block
-    const Img m = img_at(I, img_of(I, gr, RowBase()));
-    const int y = gr - m.row_base;
-    long long key = -1;
-    Fix128 v = {0ull, 0ll};
-    if (x < m.W) {
-      const int32_t p = px<int32_t>(m.aux, m.pitch, y, x);
-      if (p != INT_MIN) {
-        const int64_t q = p >= 0 ? (int64_t)p : ~(int64_t)p;
-        if (q < (int64_t)m.H * m.W && fix_from_float(px<float>(m.plane, m.pitch, y, x), v)) {
-          key = ((int64_t)m.px_base + q) | (p < 0 ? (1ll << 40) : 0ll);
-        } else {
-          set_status(status, NSGB_ERR_BAD_ARG);
-          v = Fix128{0ull, 0ll};
-        }
-      }
-    }
-    const long long kprev = __shfl_up_sync(NSGB_FULL, key, 1);
-    const long long knext = __shfl_down_sync(NSGB_FULL, key, 1);
-    bool head = lane == 0 || kprev != key;
+// The adjoint: grad(q) = exact sum of the gradients of the pixels whose source is q, rounded once.
+// Sources are near their pixels (a plateau grows a few pixels around its source), so the sums are
+// formed per 32 x 32 tile in shared memory by the CTA that owns the sources, and only pixels whose
+// source lies in another tile go through 128-bit accumulators in the workspace:
+//   (1) grad_touch: the accumulators such pixels use are zeroed and marked in a bitmap;
+//   (2) grad_far: such pixels add to them (two 64-bit atomics each, runs of one row summed first);
+//   (3) grad_tiles: every tile sums its own pixels, adds the marked accumulators, rounds, writes;
+//   (4) grad_wide_tiles: the same for tiles whose gradients span too many bits for (3).
+// An accumulator for every pixel, zeroed, added to and read back (64 bytes of traffic a pixel
+// against the 16 that come in and go out), took 2.1 ms at 16 x 2048^2; this takes 0.9 ms.
+struct GradArgs {
+  const float* g;
+  const int32_t* prov;
+  float *dmarker, *dmask;
+  int64_t pitch, stride;  // bytes, of all planes
+  int H, W, n;            // images of H x W
+  int tiles_x, tiles_y;
+  unsigned div_mul;  // y = umulhi(q, div_mul) >> div_shift for q = y * W + x < 2^31 (W > 1)
+  int div_shift;
+  unsigned long long *acc[2];  // two words per pixel: marker sources, mask sources
+  unsigned* far_bits[2];       // sources with pixels in other tiles
+  int* wide;                   // [0] tiles left to grad_wide_tiles, then their indices
+  int* status;
+};
+
+template <typename T>
+__device__ __forceinline__ T* grad_row(const GradArgs& a, T* base, int img, int y) {
+  return (T*)((char*)base + img * a.stride + (int64_t)y * a.pitch);
+}
+
+// Source of a pixel: class 0 (marker q) or 1 (mask q), -1 for none (ring, or out of range: reported).
+struct GradSource {
+  int cls, q, y, x;
+};
+__device__ __forceinline__ GradSource grad_source(const GradArgs& a, int32_t p) {
+  GradSource s = {-1, 0, 0, 0};
+  if (p == INT_MIN) return s;
+  s.q = p >= 0 ? p : ~p;
+  if ((int64_t)s.q >= (int64_t)a.H * a.W) return s;
+  s.cls = p >= 0 ? 0 : 1;
+  s.y = a.W > 1 ? (int)(__umulhi((unsigned)s.q, a.div_mul) >> a.div_shift) : s.q;
+  s.x = s.q - s.y * a.W;
+  return s;
+}
+
+constexpr int kGradTile = 32;
+__device__ __forceinline__ bool other_tile(const GradSource& s, int y, int x) {
+  return ((s.y ^ y) | (s.x ^ x)) >= kGradTile;
+}
+
+// Four pixels per thread (grid: columns, rows, images).
+template <bool VEC>
+__global__ void __launch_bounds__(128) grad_touch_kernel(GradArgs a) {
+  const int x = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (x >= a.W) return;
+  for (int img = blockIdx.z; img < a.n; img += gridDim.z) {
+    for (int y = blockIdx.y; y < a.H; y += gridDim.y) {
+      const int32_t* row = grad_row(a, a.prov, img, y) + x;
+      int32_t p[4];
+      if (VEC && x + 4 <= a.W) {
+        const int4 v = __ldg((const int4*)row);
+        p[0] = v.x, p[1] = v.y, p[2] = v.z, p[3] = v.w;
+      } else {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      Fix128 v2;
-      v2.lo = __shfl_up_sync(NSGB_FULL, v.lo, o);
-      v2.hi = __shfl_up_sync(NSGB_FULL, v.hi, o);
-      const bool h2 = __shfl_up_sync(NSGB_FULL, head, o);
-      if (lane >= o && !head) {
-        v = fix_add(v, v2);
-        head = h2;
+        for (int k = 0; k < 4; ++k) p[k] = x + k < a.W ? __ldg(row + k) : INT_MIN;
       }
-    }
-    const bool tail = lane == 31 || knext != key;
-    if (tail && key >= 0) {
-      unsigned long long* a = ((key >> 40) ? acc_mask : acc_marker) + 2 * (key & ((1ll << 40) - 1));
-      const unsigned long long old = atomicAdd(a, v.lo);
-      const unsigned long long carry = old + v.lo < old ? 1ull : 0ull;
-      atomicAdd(a + 1, (unsigned long long)v.hi + carry);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const GradSource s = grad_source(a, p[k]);
+        if (s.cls < 0 || !other_tile(s, y, x + k) || (k > 0 && p[k] == p[k - 1] && (x + k) % kGradTile)) continue;
+        const int64_t gq = (int64_t)img * a.H * a.W + s.q;
+        const unsigned bit = 1u << (gq & 31);
+        unsigned* word = a.far_bits[s.cls] + (gq >> 5);
+        if (__ldcg(word) & bit) continue;  // set after its accumulator was zeroed, or about to be
+        *(ulonglong2*)(a.acc[s.cls] + 2 * gq) = make_ulonglong2(0ull, 0ull);
+        atomicOr(word, bit);
+      }
     }
   }
 }
 
-// Adjoint, pass 2: accumulators to float, one rounding each.  plane = g; dmarker / dmask at
-// byte offsets.
-__global__ void grad_out_kernel(Imgs I, int total_rows, const unsigned long long* __restrict__ acc_marker,
-                                const unsigned long long* __restrict__ acc_mask, int64_t dmarker_off,
-                                int64_t dmask_off) {
-  ccl::for_batch_quads(I, total_rows, [&](const Img& m, int y, int x, int n) {
-    const int64_t gi = (int64_t)m.px_base + (int64_t)y * m.W + x;
-    float* dm = pxp<float>((void*)shifted(m.plane, dmarker_off), m.pitch, y, x);
-    float* dk = pxp<float>((void*)shifted(m.plane, dmask_off), m.pitch, y, x);
-    float a[4], b[4];
+// Lanes of a warp hold consecutive pixels of one row, which mostly share a source: a segmented
+// warp scan sums runs of equal targets first, so only the last lane of each run issues the atomics
+// (low word, then the high word with the low word's carry).  Four rows per thread, their sources
+// loaded together; a warp without a far pixel in a row skips the row.
+constexpr int kFarRows = 4;
+__global__ void __launch_bounds__(128) grad_far_kernel(GradArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int img = blockIdx.z; img < a.n; img += gridDim.z) {
+    for (int y0 = blockIdx.y * kFarRows; y0 < a.H; y0 += gridDim.y * kFarRows) {  // uniform per block
+      int32_t p[kFarRows];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k < n) {
-        const ulonglong2 am = __ldcs((const ulonglong2*)(acc_marker + 2 * (gi + k)));
-        const ulonglong2 ak = __ldcs((const ulonglong2*)(acc_mask + 2 * (gi + k)));
-        a[k] = fix_to_float(am.x, (long long)am.y);
-        b[k] = fix_to_float(ak.x, (long long)ak.y);
-      } else {
-        a[k] = b[k] = 0.f;
+      for (int r = 0; r < kFarRows; ++r)
+        p[r] = x < a.W && y0 + r < a.H ? __ldg(grad_row(a, a.prov, img, y0 + r) + x) : INT_MIN;
+#pragma unroll 1
+      for (int r = 0; r < kFarRows; ++r) {
+        const int y = y0 + r;
+        const int32_t pr = r == 0 ? p[0] : r == 1 ? p[1] : r == 2 ? p[2] : p[3];
+        const GradSource s = grad_source(a, pr);
+        const bool far = s.cls >= 0 && other_tile(s, y, x);
+        if (!__any_sync(NSGB_FULL, far)) continue;
+        long long key = -1;
+        Fix128 v = {0ull, 0ll};
+        if (far && fix_from_float(__ldg(grad_row(a, a.g, img, y) + x), v))
+          key = ((int64_t)img * a.H * a.W + s.q) | ((long long)s.cls << 40);
+        else
+          v = Fix128{0ull, 0ll};
+        const long long kprev = __shfl_up_sync(NSGB_FULL, key, 1);
+        const long long knext = __shfl_down_sync(NSGB_FULL, key, 1);
+        bool head = lane == 0 || kprev != key || key < 0;
+#pragma unroll 1
+        for (int o = 1; o < 32 && !__all_sync(NSGB_FULL, head); o <<= 1) {
+          Fix128 v2;
+          v2.lo = __shfl_up_sync(NSGB_FULL, v.lo, o);
+          v2.hi = __shfl_up_sync(NSGB_FULL, v.hi, o);
+          const bool h2 = __shfl_up_sync(NSGB_FULL, head, o);
+          if (lane >= o && !head) {
+            v = fix_add(v, v2);
+            head = h2;
+          }
+        }
+        const bool tail = lane == 31 || knext != key;
+        if (tail && key >= 0) {
+          unsigned long long* q = a.acc[key >> 40] + 2 * (key & ((1ll << 40) - 1));
+          const unsigned long long old = atomicAdd(q, v.lo);
+          const unsigned long long carry = old + v.lo < old ? 1ull : 0ull;
+          atomicAdd(q + 1, (unsigned long long)v.hi + carry);
+        }
       }
     }
-    if (n == 4 && (((uintptr_t)dm | (uintptr_t)dk) & 15) == 0) {
-      *(float4*)dm = make_float4(a[0], a[1], a[2], a[3]);
-      *(float4*)dk = make_float4(b[0], b[1], b[2], b[3]);
+  }
+}
+
+// A tile's pixels: position, source and gradient (kept in registers by both tile kernels).
+constexpr int kGradPx = kGradTile * kGradTile;
+constexpr int kGradThreads = 256;
+constexpr int kGradRows = kGradTile / (kGradThreads / 32);  // rows per thread
+struct GradTileAt {
+  int img, x0, y0;
+  int64_t px0;
+};
+__device__ __forceinline__ GradTileAt grad_tile_at(const GradArgs& a, int b) {
+  const int per = a.tiles_x * a.tiles_y;
+  GradTileAt t;
+  t.img = b / per;
+  const int lt = b - t.img * per, ty = lt / a.tiles_x;
+  t.x0 = (lt - ty * a.tiles_x) * kGradTile;
+  t.y0 = ty * kGradTile;
+  t.px0 = (int64_t)t.img * a.H * a.W;
+  return t;
+}
+__device__ __forceinline__ bool far_marked(const GradArgs& a, int c, int64_t gq) {
+  return (__ldg(a.far_bits[c] + (gq >> 5)) >> (gq & 31)) & 1u;
+}
+__device__ __forceinline__ Fix128 far_sum(const GradArgs& a, int c, int64_t gq) {
+  const ulonglong2 v = __ldcg((const ulonglong2*)(a.acc[c] + 2 * gq));
+  return Fix128{v.x, (long long)v.y};
+}
+
+// When the tile's non-zero gradients lie within 30 binary orders of magnitude (and above 2^-73,
+// where every bit counts), each is an integer of 53 bits at most in units of the smallest one's last
+// bit, and the sum of all 1024 fits 63 bits.  It is added to three signed 32-bit limbs of 21 bits
+// (1024 pixels cannot overflow one) without returning atomics or carries, and the total converts
+// to float with one rounding (the scale is a power of two).  Tiles outside that range are listed
+// for grad_wide_tiles.
+constexpr int kSpan = 29;
+__global__ void __launch_bounds__(kGradThreads) grad_tiles_kernel(GradArgs a) {
+  __shared__ int limb[2][3][kGradPx];
+  __shared__ uint16_t list[2 * kGradPx];  // class * kGradPx + pixel: sums with a far part
+  __shared__ int listed, s_lo[kGradThreads / 32], s_hi[kGradThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const GradTileAt T = grad_tile_at(a, blockIdx.x);
+  const int x = T.x0 + lane, yw = T.y0 + warp * kGradRows;
+  const int64_t at = T.img * a.stride + (int64_t)yw * a.pitch + (int64_t)x * 4;  // first row, bytes
+  const int rows_in = x < a.W ? min(kGradRows, a.H - yw) : 0;
+  int32_t p[kGradRows];
+  uint32_t g[kGradRows];
+  int lo = 255, hi = 0;  // exponents of the non-zero gradients
+#pragma unroll
+  for (int k = 0; k < kGradRows; ++k) {
+    p[k] = k < rows_in ? __ldg((const int32_t*)((const char*)a.prov + at + k * a.pitch)) : INT_MIN;
+    g[k] = k < rows_in ? __ldg((const uint32_t*)((const char*)a.g + at + k * a.pitch)) : 0u;
+  }
+  for (int i = threadIdx.x; i < 2 * 3 * kGradPx / 4; i += kGradThreads)
+    ((uint4*)limb)[i] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int k = 0; k < kGradRows; ++k) {
+    const int ex = (g[k] >> 23) & 0xFF;
+    if (g[k] << 1) lo = min(lo, ex), hi = max(hi, ex);
+  }
+  lo = __reduce_min_sync(NSGB_FULL, lo);
+  hi = __reduce_max_sync(NSGB_FULL, hi);
+  if (lane == 0) s_lo[warp] = lo, s_hi[warp] = hi;
+  if (threadIdx.x == 0) listed = 0;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kGradThreads / 32; ++w) lo = min(lo, s_lo[w]), hi = max(hi, s_hi[w]);
+  if (lo <= hi && (lo < 127 - 73 || hi >= 127 + 31 || hi - lo > kSpan)) {
+    if (threadIdx.x == 0) a.wide[1 + atomicAdd(a.wide, 1)] = blockIdx.x;
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < kGradRows; ++k) {
+    if (p[k] == INT_MIN) continue;
+    const GradSource s = grad_source(a, p[k]);
+    if (s.cls < 0) {
+      set_status(a.status, NSGB_ERR_BAD_ARG);
+      continue;
+    }
+    if (other_tile(s, yw + k, x) || (g[k] << 1) == 0u) continue;
+    const int i = (s.y & (kGradTile - 1)) * kGradTile + (s.x & (kGradTile - 1));
+    const unsigned long long v = (unsigned long long)((g[k] & 0x7FFFFFu) | 0x800000u) << (((g[k] >> 23) & 0xFF) - lo);
+    const int sign = (int)g[k] >> 31;  // 0 or -1
+    constexpr int kMask = (1 << 21) - 1;
+    const int l0 = (int)v & kMask, l1 = (int)(v >> 21) & kMask, l2 = (int)(v >> 42);
+    if (l0) atomicAdd(&limb[s.cls][0][i], (l0 ^ sign) - sign);
+    if (l1) atomicAdd(&limb[s.cls][1][i], (l1 ^ sign) - sign);
+    if (l2) atomicAdd(&limb[s.cls][2][i], (l2 ^ sign) - sign);
+  }
+  __syncthreads();
+  const float scale = __uint_as_float((unsigned)(min(lo, 254) - 23) << 23);  // 2^(lo - 150)
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    char* const out = (char*)(c ? a.dmask : a.dmarker) + at;
+    const unsigned* const bits = a.far_bits[c];
+#pragma unroll
+    for (int k = 0; k < kGradRows; ++k) {
+      const int i = (warp * kGradRows + k) * kGradTile + lane;
+      // the far bits of the tile's 32 pixels of this row (the bitmap has a spare word at its end)
+      const int64_t gq = T.px0 + (int64_t)min(yw + k, a.H - 1) * a.W + T.x0;
+      const unsigned* word = bits + (gq >> 5);
+      const unsigned row_far = __funnelshift_r(__ldg(word), __ldg(word + 1), (unsigned)gq & 31u);
+      const bool far = k < rows_in && ((row_far >> lane) & 1u);
+      if (k < rows_in) {
+        const long long sum = limb[c][0][i] + ((long long)limb[c][1][i] << 21) + ((long long)limb[c][2][i] << 42);
+        if (!far) *(float*)(out + k * a.pitch) = __ll2float_rn(sum) * scale;
+      }
+      const unsigned m = __ballot_sync(NSGB_FULL, far);
+      if (m) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&listed, __popc(m));
+        base = __shfl_sync(NSGB_FULL, base, 0);
+        if (far) list[base + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(c * kGradPx + i);
+      }
+    }
+  }
+  __syncthreads();
+  const int up = lo <= hi ? lo - 150 + 96 : 0;  // the tile's unit is 2^(up - 96), 0 <= up <= 103
+  for (int j = threadIdx.x; j < listed; j += kGradThreads) {
+    const int c = list[j] / kGradPx, i = list[j] & (kGradPx - 1);
+    const int y = T.y0 + i / kGradTile, xi = T.x0 + (i & (kGradTile - 1));
+    const long long sum = limb[c][0][i] + ((long long)limb[c][1][i] << 21) + ((long long)limb[c][2][i] << 42);
+    Fix128 v;
+    if (up < 64) {
+      v.lo = (unsigned long long)sum << up;
+      v.hi = up ? sum >> (64 - up) : sum >> 63;
     } else {
-      for (int k = 0; k < n; ++k) {
-        dm[k] = a[k];
-        dk[k] = b[k];
+      v.lo = 0ull;
+      v.hi = (long long)((unsigned long long)sum << (up - 64));
+    }
+    v = fix_add(v, far_sum(a, c, T.px0 + (int64_t)y * a.W + xi));
+    grad_row(a, c ? a.dmask : a.dmarker, T.img, y)[xi] = fix_to_float(v.lo, v.hi);
+  }
+}
+
+// The listed tiles, any finite gradients below 2^31.  The first gradient a source receives stays in
+// its slot as it is; any further one is added to six signed 32-bit limbs of 21 bits (a gradient's
+// 24 bits touch three at most, and 1024 pixels cannot overflow the lower five).  Sources whose
+// limbs are not zero or that are marked in the bitmap are listed and converted densely; the others
+// are their slot.
+constexpr int kLimbs = 6, kLimbBits = 21;
+constexpr uint32_t kNoGrad = 0xFFFFFFFFu;  // a NaN: never a gradient in a slot
+struct GradTile {
+  uint32_t slot[2][kGradPx];
+  int limb[2][kLimbs][kGradPx];
+  uint16_t list[2 * kGradPx];  // class * kGradPx + pixel
+  int listed;
+};
+
+__device__ __forceinline__ void limb_add(int (*limb)[kGradPx], int i, float g) {
+  const uint32_t b = __float_as_uint(g), ex = (b >> 23) & 0xFFu;
+  uint32_t man = b & 0x7FFFFFu;
+  int s = ex == 0 ? -149 + 96 : (int)ex - 150 + 96;  // g = +-man * 2^(s - 96)
+  if (ex != 0) man |= 0x800000u;
+  if (s < 0) {  // round to the resolution, ties to even
+    const int r = -s;
+    if (r >= 32) return;
+    const uint32_t q = man >> r, rem = man & ((1u << r) - 1u), half = 1u << (r - 1);
+    man = q + ((rem > half || (rem == half && (q & 1u))) ? 1u : 0u);
+    s = 0;
+  }
+  const int k = s / kLimbBits;
+  unsigned long long v = (unsigned long long)man << (s - k * kLimbBits);
+  const bool neg = (b >> 31) != 0;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    // the last limb takes all that is left (s <= 103: bits 105 .. 126), modulo 2^32: the sum of a
+    // source is below 2^127, so the last limb's final value fits
+    const bool last = k + j == kLimbs - 1;
+    const int l = last ? (int)v : (int)(v & ((1u << kLimbBits) - 1u));
+    v = last ? 0ull : v >> kLimbBits;
+    if (l) atomicAdd(&limb[k + j][i], neg ? -l : l);
+  }
+}
+
+__device__ __forceinline__ void grad_wide_tile(const GradArgs& a, GradTile& S, int tile) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kRows = kGradRows;
+  const GradTileAt T = grad_tile_at(a, tile);
+  const int img = T.img, y0 = T.y0, x = T.x0 + lane;
+  const int64_t px0 = T.px0;
+  int32_t p[kRows];
+  float g[kRows];
+#pragma unroll
+  for (int k = 0; k < kRows; ++k) {
+    const int y = y0 + warp * kRows + k;
+    const bool in = y < a.H && x < a.W;
+    p[k] = in ? __ldg(grad_row(a, a.prov, img, y) + x) : INT_MIN;
+    g[k] = in ? __ldg(grad_row(a, a.g, img, y) + x) : 0.f;
+  }
+  for (int i = threadIdx.x; i < 2 * kGradPx / 4; i += kGradThreads)
+    ((uint4*)S.slot)[i] = make_uint4(kNoGrad, kNoGrad, kNoGrad, kNoGrad);
+  for (int i = threadIdx.x; i < 2 * kLimbs * kGradPx / 4; i += kGradThreads)
+    ((uint4*)S.limb)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (threadIdx.x == 0) S.listed = 0;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kRows; ++k) {
+    const int y = y0 + warp * kRows + k;
+    if (p[k] == INT_MIN) continue;
+    const GradSource s = grad_source(a, p[k]);
+    const bool bad = (__float_as_uint(g[k]) & 0x7FFFFFFFu) >= (127u + 31u) << 23;  // |g| >= 2^31, inf, NaN
+    if (s.cls < 0 || bad) {
+      set_status(a.status, NSGB_ERR_BAD_ARG);
+      continue;
+    }
+    if (other_tile(s, y, x)) continue;
+    const int i = (s.y & (kGradTile - 1)) * kGradTile + (s.x & (kGradTile - 1));
+    if (atomicCAS(&S.slot[s.cls][i], kNoGrad, __float_as_uint(g[k])) != kNoGrad) limb_add(S.limb[s.cls], i, g[k]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    float* const out = c ? a.dmask : a.dmarker;
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+      const int i = (warp * kRows + k) * kGradTile + lane;
+      const int y = y0 + warp * kRows + k;
+      const bool in = y < a.H && x < a.W;
+      int any = 0;
+#pragma unroll
+      for (int l = 0; l < kLimbs; ++l) any |= S.limb[c][l][i];
+      const uint32_t first = S.slot[c][i];
+      bool more = any != 0;
+      if (in) {
+        const int64_t gq = px0 + (int64_t)y * a.W + x;
+        more = more || far_marked(a, c, gq);
+        // a gradient below 2^-73 still has to be rounded to the resolution
+        const uint32_t mag = first == kNoGrad ? 0u : first & 0x7FFFFFFFu;
+        if (mag != 0u && mag < (127u - 73u) << 23) more = true;
+        if (!more) grad_row(a, out, img, y)[x] = mag == 0u ? 0.f : __uint_as_float(first);
+      }
+      const unsigned m = __ballot_sync(NSGB_FULL, in && more);
+      if (m) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&S.listed, __popc(m));
+        base = __shfl_sync(NSGB_FULL, base, 0);
+        if (in && more) S.list[base + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(c * kGradPx + i);
       }
     }
-  });
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < S.listed; j += kGradThreads) {
+    const int c = S.list[j] / kGradPx, i = S.list[j] & (kGradPx - 1);
+    const int y = y0 + i / kGradTile, xi = T.x0 + (i & (kGradTile - 1));
+    __int128 sum = 0;
+#pragma unroll
+    for (int l = kLimbs - 1; l >= 0; --l) sum = sum * (1 << kLimbBits) + S.limb[c][l][i];
+    Fix128 v = {(unsigned long long)sum, (long long)(sum >> 64)};
+    const uint32_t first = S.slot[c][i];
+    Fix128 f;
+    if (first != kNoGrad && fix_from_float(__uint_as_float(first), f)) v = fix_add(v, f);
+    const int64_t gq = px0 + (int64_t)y * a.W + xi;
+    if (far_marked(a, c, gq)) v = fix_add(v, far_sum(a, c, gq));
+    grad_row(a, c ? a.dmask : a.dmarker, img, y)[xi] = fix_to_float(v.lo, v.hi);
+  }
+}
+
+__global__ void __launch_bounds__(kGradThreads) grad_wide_tiles_kernel(GradArgs a) {
+  extern __shared__ __align__(16) unsigned char grad_smem[];
+  const int n = __ldcg(a.wide);
+  for (int j = blockIdx.x; j < n; j += gridDim.x) {
+    grad_wide_tile(a, *reinterpret_cast<GradTile*>(grad_smem), __ldcg(a.wide + 1 + j));
+    __syncthreads();
+  }
 }
 
 // Image table of `n` equally sized images `stride` bytes apart (image 0 = proto).
@@ -1782,9 +2097,15 @@ size_t f32_fwd_bytes(int64_t batch, int64_t rows, int64_t cols) {
   return ws_sizes(stacked_totals(P1.t, batch)).total;
 }
 
+int64_t grad_tiles(int64_t batch, int64_t rows, int64_t cols) {
+  return batch * ((rows + kGradTile - 1) / kGradTile) * ((cols + kGradTile - 1) / kGradTile);
+}
+
 size_t f32_bwd_bytes(int64_t batch, int64_t rows, int64_t cols) {
+  // status, the accumulators and bitmaps of marker and mask sources, the list of wide tiles
   const size_t px = (size_t)(batch * rows * cols);
-  return 256 + 2 * align256(16 * px) + (batch > 1 ? align256(sizeof(Img) * (size_t)batch) : 0);
+  return 256 + 2 * align256(16 * px) + 2 * align256(sizeof(unsigned) * (px / 32 + 2)) +
+         align256(sizeof(int) * (size_t)(grad_tiles(batch, rows, cols) + 1));
 }
 
 // Plan over the stacked images; with more than one image the table is built on the device.
@@ -1855,20 +2176,48 @@ nsgb_status nsgb_recon_f32_bwd(const float* grad_out, const int32_t* prov, float
   if (st != NSGB_OK) return st;
   cudaStream_t s = (cudaStream_t)stream;
   const size_t px = (size_t)(batch * rows * cols);
+  const size_t acc_bytes = align256(16 * px), bit_bytes = align256(sizeof(unsigned) * (px / 32 + 2));
   char* p = (char*)ws;
-  int* status = (int*)p;
-  auto* am = (unsigned long long*)(p + 256);
-  auto* ak = (unsigned long long*)(p + 256 + align256(16 * px));
-  Img* table = batch > 1 ? (Img*)(p + 256 + 2 * align256(16 * px)) : nullptr;
-  Plan P;
-  cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(am, 0, 2 * align256(16 * px), s);
-  if (e == cudaSuccess) e = stacked_plan((void*)grad_out, prov, batch, rows, cols, pitch, image_stride, table, &P, s);
+  GradArgs a = {};
+  a.g = grad_out;
+  a.prov = prov;
+  a.dmarker = grad_marker;
+  a.dmask = grad_mask;
+  a.pitch = pitch;
+  a.stride = batch > 1 ? image_stride : 0;
+  a.H = (int)rows;
+  a.W = (int)cols;
+  a.n = (int)batch;
+  a.tiles_x = (a.W + kGradTile - 1) / kGradTile;
+  a.tiles_y = (a.H + kGradTile - 1) / kGradTile;
+  // floor(q / W) for q < 2^31: with 2^l >= W the multiplier exceeds 2^(31 + l) / W by at most 1,
+  // which moves the quotient by q / 2^(31 + l) < 1 / W
+  int l = 0;
+  while ((1ll << l) < cols) ++l;
+  a.div_shift = l - 1;
+  a.div_mul = cols > 1 ? (unsigned)((1ull << (31 + l)) / (unsigned long long)cols + 1ull) : 0u;
+  a.status = (int*)p;
+  a.acc[0] = (unsigned long long*)(p + 256);
+  a.acc[1] = (unsigned long long*)(p + 256 + acc_bytes);
+  a.far_bits[0] = (unsigned*)(p + 256 + 2 * acc_bytes);
+  a.far_bits[1] = (unsigned*)(p + 256 + 2 * acc_bytes + bit_bytes);
+  a.wide = (int*)(p + 256 + 2 * acc_bytes + 2 * bit_bytes);
+  const bool vec = ((uintptr_t)prov % 16) == 0 && pitch % 16 == 0 && a.stride % 16 == 0;
+  cudaError_t e = cudaMemsetAsync(a.status, 0, sizeof(int), s);
+  // the bitmaps and the count of wide tiles behind them
+  if (e == cudaSuccess) e = cudaMemsetAsync(a.far_bits[0], 0, 2 * bit_bytes + sizeof(int), s);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(grad_wide_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradTile));
   if (e == cudaSuccess) {
-    grad_scatter_kernel<<<rcb(P.t), 256, 0, s>>>(P.I, P.t.rows, am, ak, status);
-    const int64_t dmo = (int64_t)((uintptr_t)grad_marker - (uintptr_t)grad_out);
-    const int64_t dko = (int64_t)((uintptr_t)grad_mask - (uintptr_t)grad_out);
-    grad_out_kernel<<<qrb(P.t), 256, 0, s>>>(P.I, P.t.rows, am, ak, dmo, dko);
+    const unsigned gy = (unsigned)std::min<int64_t>(rows, 65535), gz = (unsigned)std::min<int64_t>(batch, 65535);
+    const dim3 quads((a.W + 511) / 512, gy, gz);
+    const dim3 rows4((a.W + 127) / 128, (unsigned)std::min<int64_t>((rows + kFarRows - 1) / kFarRows, 65535), gz);
+    const int64_t tiles = grad_tiles(batch, rows, cols);
+    if (vec) grad_touch_kernel<true><<<quads, 128, 0, s>>>(a);
+    else grad_touch_kernel<false><<<quads, 128, 0, s>>>(a);
+    grad_far_kernel<<<rows4, 128, 0, s>>>(a);
+    grad_tiles_kernel<<<(unsigned)tiles, kGradThreads, 0, s>>>(a);
+    grad_wide_tiles_kernel<<<(unsigned)std::min<int64_t>(tiles, 3 * 152), kGradThreads, sizeof(GradTile), s>>>(a);
     e = cudaGetLastError();
   }
   return finish(e, ws, s, opts);
