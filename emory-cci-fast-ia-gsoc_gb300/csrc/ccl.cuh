@@ -51,6 +51,7 @@ __device__ __forceinline__ bool joins_diagonally(uint32_t c) {
   else return c == 2u;
 }
 constexpr int kLocalWarps = 4;  // labelling tiles (one warp each) per CTA of ccl_local
+constexpr int kMergeTiles = 4;  // labelling tiles (two warps each) per CTA of ccl_merge
 
 // Tile-local forest of one warp (shared memory, 1024 words).  Node i = 32 * row + column; its
 // word sits at s[i ^ (i >> 5)], so the same column of 32 rows lies in 32 banks.  A word holds the
@@ -132,11 +133,14 @@ __device__ __forceinline__ void g_union(int* L, int a, int b) {
 // root is px_base + the smallest raster index of the component.  A (optional) holds the pixel
 // count of each local root, then of each global root.  `roots` lists the local roots,
 // `nroots` counts them.
+// `skip` (optional): a device word; while it is not zero the labelling kernels return at once.
 struct Forest {
   int* L;
   int* A;
   int* roots;
   int* nroots;
+  const int* skip = nullptr;
+  __device__ bool skipped() const { return skip && __ldcg(skip) != 0; }
 };
 
 __device__ __forceinline__ int root_of(const int* L, int64_t i) {
@@ -272,7 +276,7 @@ __global__ void __launch_bounds__(32 * kLocalWarps) ccl_local(Cls cls, Imgs I, F
   __shared__ int s_nodes[kLocalWarps][kTile * kTile];
   __shared__ unsigned s_starts[kLocalWarps][kTile];
   const int b = blockIdx.x * kLocalWarps + (threadIdx.x >> 5);
-  if (b >= ntiles) return;  // whole warp; the warps of a CTA are independent
+  if (b >= ntiles || f.skipped()) return;  // whole warp; the warps of a CTA are independent
   int* s = s_nodes[threadIdx.x >> 5];
   unsigned* starts = s_starts[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -450,13 +454,17 @@ __global__ void __launch_bounds__(32 * kLocalWarps) ccl_local(Cls cls, Imgs I, F
 // where a run on the far side starts or where a near-side run starts under a far-side run,
 // plus the two diagonal ends of each far-side run for 8-connectivity.
 template <class Cls, int CONN>
-__global__ void __launch_bounds__(64) ccl_merge(Cls cls, Imgs I, int* __restrict__ L) {
+__global__ void __launch_bounds__(64 * kMergeTiles) ccl_merge(Cls cls, Imgs I, Forest f, int ntiles) {
   pdl_wait();
   pdl_release();
-  const TileAt T = tile_at(I, blockIdx.x);
+  if (f.skipped()) return;
+  int* __restrict__ const L = f.L;
+  const int b = blockIdx.x * kMergeTiles + (threadIdx.x >> 6);
+  if (b >= ntiles) return;
+  const TileAt T = tile_at(I, b);
   const int x0 = T.x0, y0 = T.y0, H = T.m.H, W = T.m.W, pb = T.m.px_base;
   const int lane = threadIdx.x & 31;
-  const bool bottom = (threadIdx.x >> 5) == 0;
+  const bool bottom = ((threadIdx.x >> 5) & 1) == 0;
   // coordinates of the near pixel (a) and the far pixel (b) for this lane
   int ay, ax, by, bx;
   if (bottom) {
@@ -717,6 +725,7 @@ inline dim3 quadrow_grid(int total_rows, int max_w) {
   return dim3(bx, row_blocks(total_rows));
 }
 
+inline unsigned merge_grid(int c_tiles) { return (unsigned)((c_tiles + kMergeTiles - 1) / kMergeTiles); }
 inline unsigned local_grid(int c_tiles) { return (unsigned)((c_tiles + kLocalWarps - 1) / kLocalWarps); }
 
 // Labels every image of the batch: local pass, edge merge, root flattening.  Afterwards
@@ -727,10 +736,10 @@ cudaError_t label(const Cls& cls, const Imgs& I, const BatchTotals& t, int conn,
   if (e != cudaSuccess) return e;
   if (conn == 8) {
     ccl_local<Cls, 8><<<local_grid(t.c_tiles), 32 * kLocalWarps, 0, s>>>(cls, I, f, t.c_tiles);
-    ccl_merge<Cls, 8><<<t.c_tiles, 64, 0, s>>>(cls, I, f.L);
+    ccl_merge<Cls, 8><<<merge_grid(t.c_tiles), 64 * kMergeTiles, 0, s>>>(cls, I, f, t.c_tiles);
   } else {
     ccl_local<Cls, 4><<<local_grid(t.c_tiles), 32 * kLocalWarps, 0, s>>>(cls, I, f, t.c_tiles);
-    ccl_merge<Cls, 4><<<t.c_tiles, 64, 0, s>>>(cls, I, f.L);
+    ccl_merge<Cls, 4><<<merge_grid(t.c_tiles), 64 * kMergeTiles, 0, s>>>(cls, I, f, t.c_tiles);
   }
   ccl_flatten_roots<<<list_grid(t.px), 256, 0, s>>>(f, (int)t.px);
   return cudaGetLastError();
@@ -818,10 +827,10 @@ cudaError_t label_filled(const Cls& cls, const Imgs& I, const BatchTotals& t, in
   if (e != cudaSuccess) return e;
   if (conn == kConnFg8Bg4) {
     e = launch_k(pdl, ccl_local<Cls, kConnFg8Bg4>, dim3(local_grid(t.c_tiles)), dim3(32 * kLocalWarps), s, cls, I, f, t.c_tiles);
-    if (e == cudaSuccess) e = launch_k(pdl, ccl_merge<Cls, kConnFg8Bg4>, dim3(t.c_tiles), dim3(64), s, cls, I, f.L);
+    if (e == cudaSuccess) e = launch_k(pdl, ccl_merge<Cls, kConnFg8Bg4>, dim3(merge_grid(t.c_tiles)), dim3(64 * kMergeTiles), s, cls, I, f, t.c_tiles);
   } else {
     e = launch_k(pdl, ccl_local<Cls, kConnFg4Bg8>, dim3(local_grid(t.c_tiles)), dim3(32 * kLocalWarps), s, cls, I, f, t.c_tiles);
-    if (e == cudaSuccess) e = launch_k(pdl, ccl_merge<Cls, kConnFg4Bg8>, dim3(t.c_tiles), dim3(64), s, cls, I, f.L);
+    if (e == cudaSuccess) e = launch_k(pdl, ccl_merge<Cls, kConnFg4Bg8>, dim3(merge_grid(t.c_tiles)), dim3(64 * kMergeTiles), s, cls, I, f, t.c_tiles);
   }
   const int gx = (t.perimeter_max + 255) / 256 > 64 ? 64 : (t.perimeter_max + 255) / 256;
   if (e == cudaSuccess)
