@@ -214,10 +214,6 @@ __device__ __forceinline__ void flood_visit(const FloodArgs& a, int t, int lane)
       break;
     }
   }
-  if (lane == 0) {
-    atomicAdd(&a.c.stats[0], 1);
-    atomicAdd(&a.c.stats[1], it);
-  }
   if (__any_sync(NSGB_FULL, any != 0) && col_in) {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
@@ -254,23 +250,15 @@ __device__ __forceinline__ void flood_visit(const FloodArgs& a, int t, int lane)
       if ((c1 >> 31) && ((HRp & ~HRf) >> 33) & 1ull) dirs |= 1u << 8;
     }
   }
-  // The warp barrier orders every lane's stores before the release atomics below.
+  // The warp barrier orders every lane's stores before the fence below.
   __syncwarp();
-  if (lane < 9 && ((dirs >> lane) & 1u)) {
-    const int ny = ty + lane / 3 - 1, nx = tx + lane % 3 - 1;
-    if (ny >= 0 && ny < nty && nx >= 0 && nx < ntx) mark_tile(a.c, (I.d ? m.f_tile_base : 0) + ny * ntx + nx);
-  }
-  __syncwarp();
+  const int ny = ty + lane / 3 - 1, nx = tx + lane % 3 - 1;
+  const bool mark = lane < 9 && ((dirs >> lane) & 1u) && ny >= 0 && ny < nty && nx >= 0 && nx < ntx;
+  mark_and_release(a.c, mark, (I.d ? m.f_tile_base : 0) + ny * ntx + nx, t, lane);
   if (lane == 0) {
-    if (atom_cas_acq_rel(&a.c.state[t], kRunning, kIdle) == kRunning) {
-      pending_release(a.c);
-    } else {
-      atom_exch_acq_rel(&a.c.state[t], kQueued);
-      atomicAdd(&a.c.stats[2], 1);
-      queue_push(a.c, t);
-    }
+    atomicAdd(&a.c.stats[0], 1);
+    atomicAdd(&a.c.stats[1], it);
   }
-  __syncwarp();
 }
 
 template <int CONN>
@@ -315,8 +303,7 @@ __global__ void flood_seed_finish_kernel(Ctl c, const unsigned* counter) {
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *c.head = 0u;
-    *c.tail = n;
-    *c.pending = (int)n;
+    *c.tally = Tally{(int)n, n};
     if (n == 0) *c.done = 1;
   }
 }
@@ -337,8 +324,7 @@ cudaError_t flood_launch(const Imgs& I, int ntiles, const uint32_t* open, uint32
   a.c.visit_count = (unsigned long long*)(wi + 6);
   a.c.prof = (unsigned long long*)(wi + 160);
   a.c.head = (unsigned*)(wi + 32);
-  a.c.tail = (unsigned*)(wi + 64);
-  a.c.pending = wi + 96;
+  a.c.tally = (Tally*)(wi + 64);
   a.c.done = wi + 128;
   a.c.state = wi + kFloodHdrInts;
   a.c.cap = ring_cap(ntiles);

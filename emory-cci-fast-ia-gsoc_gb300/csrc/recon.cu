@@ -59,7 +59,7 @@ struct alignas(16) WarpBuf {
   uint32_t mv[32 * kS];  // mask, column-pass layout [lane*kS + i]
   uint32_t lv[36], rv[36];  // halo columns (values), index r + 1 for rows r = -1 .. 32
   uint32_t lm[36], rm[36];  // halo columns (masks)
-  uint32_t c0[32], c1[32];  // final first / last tile column, for the neighbour test
+  uint32_t c0[32], c1[32];  // first / last tile column after the last row pass, for the neighbour test
   uint32_t hl[32], hr[32];  // per row: what the halo columns give the first / last column
 };
 
@@ -333,7 +333,7 @@ __device__ __forceinline__ uint32_t tile_sum(const uint32_t (&O)[32]) {
 // and against the constant halo carries).  If the pass changes nothing, its seam inputs were the
 // final values, so it is exact as well.  TRACK: return the xor / or change word.
 template <typename T, bool TRACK>
-__device__ __forceinline__ uint32_t row_pass(uint32_t (&O)[32], const uint32_t* mh, const WarpBuf& B, int lane,
+__device__ __forceinline__ uint32_t row_pass(uint32_t (&O)[32], const uint32_t* mh, WarpBuf& B, int lane,
                                              bool& exact) {
   using P = Px<T>;
   uint32_t acc = 0;
@@ -370,6 +370,8 @@ __device__ __forceinline__ uint32_t row_pass(uint32_t (&O)[32], const uint32_t* 
     const uint32_t other = __shfl_xor_sync(NSGB_FULL, own, 16);
     const uint32_t own_m = mh[lane * kS + (half ? 0 : 31)];
     exact = !__any_sync(NSGB_FULL, P::vmax(own, P::vmin(other, own_m)) != own);
+    const uint32_t edge = half ? O[31] : O[0];  // the tile's last / first column, two rows
+    sts2((half ? B.c1 : B.c0) + 2 * q, P::elem(edge, 0), P::elem(edge, 1));
   } else {
     uint32_t v = B.hl[lane];
 #pragma unroll
@@ -393,6 +395,8 @@ __device__ __forceinline__ uint32_t row_pass(uint32_t (&O)[32], const uint32_t* 
       O[j + 1] = n1;
       v = n0;
     }
+    B.c0[lane] = O[0];
+    B.c1[lane] = O[31];
     exact = true;
   }
   return acc;
@@ -678,7 +682,7 @@ __device__ __forceinline__ void visit(const Args& a, WarpBuf& B, int t, int lane
   // Mask in the row layout.
   if constexpr (E == 2) {
     const int q = lane & 15, half = lane >> 4;
-#pragma unroll
+#pragma unroll 4
     for (int j = 0; j < 32; j += 2) {
       const uint2 m = lds2(B.mv + (16 * half + (j >> 1)) * kS + 2 * q);
       sts2(B.mh + lane * kS + j, __byte_perm(m.x, m.y, 0x5410), __byte_perm(m.x, m.y, 0x7632));
@@ -739,15 +743,7 @@ __device__ __forceinline__ void visit(const Args& a, WarpBuf& B, int t, int lane
   }
   {
     // first / last columns against the halo columns
-    if (lane == 0) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) B.c0[i] = P::elem(O[i], 0);
-    }
-    if (lane == 31) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) B.c1[i] = P::elem(O[i], E - 1);
-    }
-    __syncwarp();
+    // (written by the last row pass: the column pass after it changed nothing, or there was none)
     const int r = lane;
     uint32_t cl = B.c0[r], cr = B.c1[r];
     if constexpr (CONN == 8) {
@@ -771,58 +767,68 @@ __device__ __forceinline__ void visit(const Args& a, WarpBuf& B, int t, int lane
       if (P::lt(B.rv[33], P::emin(B.c1[31], B.rm[33]))) dirs |= 1u << 8;
     }
   }
-  // The warp barrier orders every lane's stores before the release atomics below.
+  // The warp barrier orders every lane's stores before the fence below.
   __syncwarp();
   PROF_MARK(5);
-  // Lane d marks the neighbour in direction d (one copy of the marking code, up to eight
-  // neighbours marked in parallel).
-  if (lane < 9 && ((dirs >> lane) & 1u)) {
-    const int ny = ty + lane / 3 - 1, nx = tx + lane % 3 - 1;
-    if (ny >= 0 && ny < IMF(r_tiles_y) && nx >= 0 && nx < IMF(r_tiles_x))
-      mark_tile(a.c, IMF(r_tile_base) + ny * IMF(r_tiles_x) + nx);
-  }
-  __syncwarp();
-  PROF_MARK(6);
-
-  // Release the tile.  If a neighbour changed while it ran, only its halo can be stale (no
+  // Mark the neighbours (lane d the one in direction d) and release the tile.  If a neighbour
+  // changed while it ran, only its halo can be stale (no
   // other warp writes its pixels).  Up to `resweeps` times the warp then takes the tile back,
   // reloads just the halo and sweeps again from the values in its registers; otherwise the
   // tile goes to the back of the queue, so that the neighbours still running finish first.
   // Re-sweeping pays off where a front crosses the image (hole filling from the border: about
   // a third less time at 16384^2) and costs time where many neighbours run at once (the
   // h-maxima style marker of the chain: about 8% more), so the caller chooses.
-  if constexpr (!RS) {
-    // (without re-sweeps the loop body runs once: kept separate so that the compiler emits
-    // one copy of the sweep code)
+  if constexpr (E == 2 && !RS) {
+    const int ny = ty + lane / 3 - 1, nx = tx + lane % 3 - 1;
+    const bool mark = lane < 9 && ((dirs >> lane) & 1u) && ny >= 0 && ny < IMF(r_tiles_y) && nx >= 0 && nx < IMF(r_tiles_x);
+    const int nt = mark ? IMF(r_tile_base) + ny * IMF(r_tiles_x) + nx : t;
+    mark_and_release(a.c, mark, nt, t, lane);
+    PROF_MARK(6);
+    return;  // (without re-sweeps the loop body runs once)
+  } else {
+    // Lane d marks the neighbour in direction d (one copy of the marking code, up to eight
+    // neighbours marked in parallel).
+    if (lane < 9 && ((dirs >> lane) & 1u)) {
+      const int ny = ty + lane / 3 - 1, nx = tx + lane % 3 - 1;
+      if (ny >= 0 && ny < IMF(r_tiles_y) && nx >= 0 && nx < IMF(r_tiles_x))
+        mark_tile(a.c, IMF(r_tile_base) + ny * IMF(r_tiles_x) + nx);
+    }
+    __syncwarp();
+    PROF_MARK(6);
+
+    if constexpr (!RS) {
+      // (without re-sweeps the loop body runs once: kept separate so that the compiler emits
+      // one copy of the sweep code)
+      if (lane == 0) {
+        if (atom_cas_acq_rel(&a.c.state[t], kRunning, kIdle) == kRunning) {
+          pending_release(a.c);
+        } else {
+          atom_exch_acq_rel(&a.c.state[t], kQueued);
+          atomicAdd(&a.c.stats[2], 1);
+          queue_push(a.c, t, 0);
+        }
+      }
+      __syncwarp();
+      return;
+    }
+    int st = 0;
     if (lane == 0) {
       if (atom_cas_acq_rel(&a.c.state[t], kRunning, kIdle) == kRunning) {
         pending_release(a.c);
+        st = 0;
+      } else if (round < a.resweeps) {
+        atom_exch_acq_rel(&a.c.state[t], kRunning);
+        atomicAdd(&a.c.stats[3], 1);
+        st = 1;
       } else {
         atom_exch_acq_rel(&a.c.state[t], kQueued);
         atomicAdd(&a.c.stats[2], 1);
-        queue_push(a.c, t);
+        queue_push(a.c, t, 0);
+        st = 0;
       }
     }
-    __syncwarp();
-    return;
+    if (__shfl_sync(NSGB_FULL, st, 0) == 0) return;
   }
-  int st = 0;
-  if (lane == 0) {
-    if (atom_cas_acq_rel(&a.c.state[t], kRunning, kIdle) == kRunning) {
-      pending_release(a.c);
-      st = 0;
-    } else if (round < a.resweeps) {
-      atom_exch_acq_rel(&a.c.state[t], kRunning);
-      atomicAdd(&a.c.stats[3], 1);
-      st = 1;
-    } else {
-      atom_exch_acq_rel(&a.c.state[t], kQueued);
-      atomicAdd(&a.c.stats[2], 1);
-      queue_push(a.c, t);
-      st = 0;
-    }
-  }
-  if (__shfl_sync(NSGB_FULL, st, 0) == 0) return;
   // the acquire exchange above orders reading the halo again after the markers' stores
   __syncwarp();
   {
@@ -974,7 +980,7 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, WarpBuf& B, int t, 
   halo_carries<T, CONN>(B, lane);
   if constexpr (E == 2) {
     const int q = lane & 15, half = lane >> 4;
-#pragma unroll
+#pragma unroll 4
     for (int j = 0; j < 32; j += 2) {
       const uint2 mm = lds2(B.mv + (16 * half + (j >> 1)) * kS + 2 * q);
       sts2(B.mh + lane * kS + j, __byte_perm(mm.x, mm.y, 0x5410), __byte_perm(mm.x, mm.y, 0x7632));
@@ -1023,15 +1029,6 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, WarpBuf& B, int t, 
       if (__any_sync(NSGB_FULL, P::vmax(botv, c_bot) != botv)) dirs |= 1u << 7;
     }
     {
-      if (lane == 0) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) B.c0[i] = P::elem(O[i], 0);
-      }
-      if (lane == 31) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) B.c1[i] = P::elem(O[i], E - 1);
-      }
-      __syncwarp();
       const int r = lane;
       uint32_t cl = B.c0[r], cr = B.c1[r];
       if constexpr (CONN == 8) {
@@ -1098,8 +1095,7 @@ __global__ void recon_seed_finish_kernel(Ctl c, const unsigned* counter, unsigne
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *c.head = 0u;
-    *c.tail = n;
-    *c.pending = (int)n;
+    *c.tally = Tally{(int)n, n};
     *c.visit_count = pass_visits;
     if (pass_visits > (unsigned long long)c.max_visits) set_status(c.status, kDevNotConverged);
     if (n == 0) *c.done = 1;
@@ -1206,16 +1202,15 @@ __global__ void recon_init_kernel(Ctl c, Imgs I, int ntiles, int order) {
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *c.head = 0u;
-    *c.tail = (unsigned)ntiles;
-    *c.pending = ntiles;
+    *c.tally = Tally{ntiles, (unsigned)ntiles};
   }
 }
 
 // Workspace layout (ints): [0] status, [1..4] stats (visits, sweeps, re-runs, re-sweeps),
 // [5] profiler visit index, [6..7] visit counter (64-bit), [8] tiles seeded by the streaming
-// passes, [32] head, [64] tail, [96] pending,
+// passes, [32] head, [64..65] pending and tail,
 // [128] done flag, [160..175] phase timers (8 x 64-bit); from int kHdrInts: state[ntiles],
-// then the ring (2 ints per slot, cap slots).  Head, tail, pending and the done flag sit on
+// then the ring (2 ints per slot, cap slots).  Head, tally and the done flag sit on
 // separate 128-byte lines: the atomics of the working warps and the polls of the waiting
 // ones then do not queue behind one another.
 constexpr int kHdrInts = 192;
@@ -1338,8 +1333,7 @@ cudaError_t launch_typed(const Imgs& I, int ntiles, bool erode, bool ring, void*
   a.c.visit_count = (unsigned long long*)(wi + 6);
   a.c.prof = (unsigned long long*)(wi + 160);
   a.c.head = (unsigned*)(wi + 32);
-  a.c.tail = (unsigned*)(wi + 64);
-  a.c.pending = wi + 96;
+  a.c.tally = (Tally*)(wi + 64);
   a.c.done = wi + 128;
   a.c.state = wi + kHdrInts;
   a.c.cap = ring_cap(ntiles);
