@@ -208,11 +208,9 @@ cudaError_t rank_roots(const Imgs& I, const BatchTotals& t, const Forest& f, int
 }
 
 cudaError_t count_roots(const Imgs& I, const BatchTotals& t, const Forest& f, int lo, int hi, unsigned* bits,
-                        int* counts, cudaStream_t s, const unsigned* skip) {
-  cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * 2 * (size_t)t.n, s);
-  if (e != cudaSuccess) return e;
-  mark_roots<<<list_grid(t.px), kRankThreads, 0, s>>>(I, f, (int)t.px, lo, hi, bits, counts, skip);
-  return cudaGetLastError();
+                        int* counts, cudaStream_t s, const unsigned* skip, bool pdl) {
+  return launch_k(pdl, mark_roots, dim3(list_grid(t.px)), dim3(kRankThreads), s, I, f, (int)t.px, lo, hi, bits, counts,
+                  skip);
 }
 
 }  // namespace ccl

@@ -621,6 +621,8 @@ __device__ __forceinline__ void roots4_ro(const int* L, int64_t i, int n, int (&
 template <class Seed>
 __global__ void ccl_seed_pixels(Imgs I, int total_rows, const int* __restrict__ L, Seed seed,
                                 unsigned* __restrict__ bits) {
+  pdl_wait();
+  pdl_release();
   for_batch_pixels(I, total_rows, [&](const Img& m, int y, int x) {
     if (!seed(m, y, x)) return;
     const int r = root_of(L, (int64_t)m.px_base + (int64_t)y * m.W + x);
@@ -633,6 +635,8 @@ __global__ void ccl_seed_pixels(Imgs I, int total_rows, const int* __restrict__ 
 template <class Seed>
 __global__ void ccl_seed_quads(Imgs I, int total_rows, const int* __restrict__ L, Seed seed,
                                unsigned* __restrict__ bits) {
+  pdl_wait();
+  pdl_release();
   for_batch_quads(I, total_rows, [&](const Img& m, int y, int x, int n) {
     bool sd[4];
     bool any = false;
@@ -671,6 +675,8 @@ __device__ __forceinline__ void border_pixel(int k, int H, int W, int& y, int& x
 // Seed pixels on each image's border only: blockIdx.y = image, x walks its border.
 template <class Seed>
 __global__ void ccl_seed_border(Imgs I, const int* __restrict__ L, Seed seed, unsigned* __restrict__ bits) {
+  pdl_wait();
+  pdl_release();
   const Img m = img_at(I, blockIdx.y);
   const int H = m.H, W = m.W;
   const int per = 2 * W + 2 * H;
@@ -728,48 +734,6 @@ inline dim3 quadrow_grid(int total_rows, int max_w) {
 inline unsigned merge_grid(int c_tiles) { return (unsigned)((c_tiles + kMergeTiles - 1) / kMergeTiles); }
 inline unsigned local_grid(int c_tiles) { return (unsigned)((c_tiles + kLocalWarps - 1) / kLocalWarps); }
 
-// Labels every image of the batch: local pass, edge merge, root flattening.  Afterwards
-// root(i) = L[L[i]].
-template <class Cls>
-cudaError_t label(const Cls& cls, const Imgs& I, const BatchTotals& t, int conn, const Forest& f, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(f.nroots, 0, sizeof(int), s);
-  if (e != cudaSuccess) return e;
-  if (conn == 8) {
-    ccl_local<Cls, 8><<<local_grid(t.c_tiles), 32 * kLocalWarps, 0, s>>>(cls, I, f, t.c_tiles);
-    ccl_merge<Cls, 8><<<merge_grid(t.c_tiles), 64 * kMergeTiles, 0, s>>>(cls, I, f, t.c_tiles);
-  } else {
-    ccl_local<Cls, 4><<<local_grid(t.c_tiles), 32 * kLocalWarps, 0, s>>>(cls, I, f, t.c_tiles);
-    ccl_merge<Cls, 4><<<merge_grid(t.c_tiles), 64 * kMergeTiles, 0, s>>>(cls, I, f, t.c_tiles);
-  }
-  ccl_flatten_roots<<<list_grid(t.px), 256, 0, s>>>(f, (int)t.px);
-  return cudaGetLastError();
-}
-
-// Enclosure tree of a two-class labelling (kConnFg8Bg4 / kConnFg4Bg8, before flattening):
-// with dual connectivities the components of the two classes form a tree by enclosure, the
-// image's outside (the components marked in `outside`, those of the outside class that touch
-// the border) at its top, and a component's parent is the component of the pixel directly
-// above its first pixel in raster order (its root).  Every component below the top joins its
-// parent, so each set that results is one component of "class 1 plus the class-2 components
-// it encloses" (class 1 with its holes filled).  One thread per listed local root; a global
-// root is hooked only by its own thread (its parent's root index is smaller than its own), so
-// the test for a global root at the start holds until the thread itself changes it.
-static __global__ void ccl_join_parents(Imgs I, Forest f, int max_roots, const unsigned* __restrict__ outside) {
-  pdl_wait();
-  pdl_release();
-  const int n = min(__ldcg(f.nroots), max_roots);
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const int r = __ldcg(f.roots + k);
-    if (ld_relaxed(f.L + r) != r) continue;
-    if ((__ldcg(outside + (r >> 5)) >> (r & 31)) & 1u) continue;
-    const Img m = img_at(I, img_of(I, r, PxBase()));
-    if (r - m.px_base < m.W) continue;  // first row: its parent is the outside
-    const int p = g_find(f.L, r - m.W);
-    if (p < 0 || ((__ldcg(outside + (p >> 5)) >> (p & 31)) & 1u)) continue;
-    g_union(f.L, r, p);
-  }
-}
-
 // Up to four word ranges to clear in one launch (n[k] words from p[k]; unused ranges have n 0).
 struct ZeroSpans {
   unsigned* p[4];
@@ -796,6 +760,55 @@ inline cudaError_t launch_k(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 
   if (pdl) return launch_dependent(kernel, grid, block, s, std::forward<Args>(args)...);
   kernel<<<grid, block, 0, s>>>(std::forward<Args>(args)...);
   return cudaGetLastError();
+}
+
+// Labels every image of the batch: local pass, edge merge, root flattening.  Afterwards
+// root(i) = L[L[i]].  The first launch is an ordinary one (it may follow anything); it clears the
+// root count and the caller's ranges 1 to 3 of `more`, so that no memset stands between the
+// launches, and every later launch is a programmatic dependent of the one before it.
+template <class Cls>
+cudaError_t label(const Cls& cls, const Imgs& I, const BatchTotals& t, int conn, const Forest& f, cudaStream_t s,
+                  ZeroSpans more = ZeroSpans{{nullptr, nullptr, nullptr, nullptr}, {0, 0, 0, 0}}) {
+  ZeroSpans z = more;
+  z.p[0] = (unsigned*)f.nroots;
+  z.n[0] = 1;
+  cudaError_t e = launch_k(false, zero_words, dim3(flat_grid(z.total())), dim3(256), s, z);
+  const dim3 lg(local_grid(t.c_tiles)), mg(merge_grid(t.c_tiles));
+  if (e != cudaSuccess) return e;
+  if (conn == 8) {
+    e = launch_dependent(ccl_local<Cls, 8>, lg, dim3(32 * kLocalWarps), s, cls, I, f, t.c_tiles);
+    if (e == cudaSuccess) e = launch_dependent(ccl_merge<Cls, 8>, mg, dim3(64 * kMergeTiles), s, cls, I, f, t.c_tiles);
+  } else {
+    e = launch_dependent(ccl_local<Cls, 4>, lg, dim3(32 * kLocalWarps), s, cls, I, f, t.c_tiles);
+    if (e == cudaSuccess) e = launch_dependent(ccl_merge<Cls, 4>, mg, dim3(64 * kMergeTiles), s, cls, I, f, t.c_tiles);
+  }
+  if (e == cudaSuccess) e = launch_dependent(ccl_flatten_roots, dim3(list_grid(t.px)), dim3(256), s, f, (int)t.px);
+  return e;
+}
+
+// Enclosure tree of a two-class labelling (kConnFg8Bg4 / kConnFg4Bg8, before flattening):
+// with dual connectivities the components of the two classes form a tree by enclosure, the
+// image's outside (the components marked in `outside`, those of the outside class that touch
+// the border) at its top, and a component's parent is the component of the pixel directly
+// above its first pixel in raster order (its root).  Every component below the top joins its
+// parent, so each set that results is one component of "class 1 plus the class-2 components
+// it encloses" (class 1 with its holes filled).  One thread per listed local root; a global
+// root is hooked only by its own thread (its parent's root index is smaller than its own), so
+// the test for a global root at the start holds until the thread itself changes it.
+static __global__ void ccl_join_parents(Imgs I, Forest f, int max_roots, const unsigned* __restrict__ outside) {
+  pdl_wait();
+  pdl_release();
+  const int n = min(__ldcg(f.nroots), max_roots);
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const int r = __ldcg(f.roots + k);
+    if (ld_relaxed(f.L + r) != r) continue;
+    if ((__ldcg(outside + (r >> 5)) >> (r & 31)) & 1u) continue;
+    const Img m = img_at(I, img_of(I, r, PxBase()));
+    if (r - m.px_base < m.W) continue;  // first row: its parent is the outside
+    const int p = g_find(f.L, r - m.W);
+    if (p < 0 || ((__ldcg(outside + (p >> 5)) >> (p & 31)) & 1u)) continue;
+    g_union(f.L, r, p);
+  }
 }
 
 // Seed test: pixels of class 2.
@@ -853,10 +866,10 @@ cudaError_t label_filled(const Cls& cls, const Imgs& I, const BatchTotals& t, in
 cudaError_t rank_roots(const Imgs& I, const BatchTotals& t, const Forest& f, int lo, int hi, int* rank,
                        unsigned* bits, size_t bits_bytes, int* block_tmp, int* wpre, int* counts, cudaStream_t s,
                        const unsigned* skip = nullptr, bool pdl = false, bool zeroed = false);
-// The counts of rank_roots alone (no ranks).  `bits` receives the global roots' bits (scratch,
-// not cleared first).
+// The counts of rank_roots alone (no ranks), into `counts` that are already clear.  `bits` receives
+// the global roots' bits (scratch, not cleared first).
 cudaError_t count_roots(const Imgs& I, const BatchTotals& t, const Forest& f, int lo, int hi, unsigned* bits,
-                        int* counts, cudaStream_t s, const unsigned* skip = nullptr);
+                        int* counts, cudaStream_t s, const unsigned* skip, bool pdl);
 constexpr int kBlockPx = 1024;
 
 // The counting half of rank_roots for any bitmap of the images' pixels: per 1024-px block the

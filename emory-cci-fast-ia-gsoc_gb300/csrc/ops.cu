@@ -210,6 +210,8 @@ __device__ __forceinline__ void store4_i32(int32_t* p, int n, const int (&v)[4])
 template <typename TO>
 __global__ void fill_out_kernel(Imgs I, int total_rows, const int* __restrict__ L, const unsigned* __restrict__ bits,
                                 uint8_t* F, TO* out, int64_t pitch_out, TO fg) {
+  pdl_wait();
+  pdl_release();
   ccl::for_batch_quads(I, total_rows, [&](const Img& m, int y, int x, int n) {
     const int64_t gi = (int64_t)m.px_base + (int64_t)y * m.W + x;
     int r[4];
@@ -290,6 +292,8 @@ __global__ void pack_open_kernel(Imgs I, int total_words, GtThr<T> gt, uint32_t*
 template <typename T>
 __global__ void binrecon_out_kernel(Imgs I, int total_rows, const int* __restrict__ L,
                                     const unsigned* __restrict__ bits) {
+  pdl_wait();
+  pdl_release();
   ccl::for_batch_pixels(I, total_rows, [&](const Img& m, int y, int x) {
     T* p = pxp<T>(m.plane, m.pitch, y, x);
     if (*p != (T)0) return;
@@ -301,6 +305,8 @@ __global__ void binrecon_out_kernel(Imgs I, int total_rows, const int* __restric
 template <typename T>
 __global__ void bwselect_out_kernel(Imgs I, int total_rows, void* out, const int* __restrict__ L,
                                     const unsigned* __restrict__ bits) {
+  pdl_wait();
+  pdl_release();
   ccl::for_batch_pixels(I, total_rows, [&](const Img& m, int y, int x) {
     const T v = px<T>(m.plane, m.pitch, y, x);
     const int r = ccl::root_of_ro(L, (int64_t)m.px_base + (int64_t)y * m.W + x);
@@ -314,6 +320,8 @@ __global__ void bwselect_out_kernel(Imgs I, int total_rows, void* out, const int
 __global__ void candidates_out_kernel(Imgs I, int total_rows, const int* __restrict__ L2,
                                       const unsigned* __restrict__ bits, const uint8_t* __restrict__ rbc,
                                       uint8_t* out) {
+  pdl_wait();
+  pdl_release();
   ccl::for_batch_quads(I, total_rows, [&](const Img& m, int y, int x, int n) {
     int r[4];
     ccl::roots4_ro(L2, (int64_t)m.px_base + (int64_t)y * m.W + x, n, r);
@@ -688,6 +696,13 @@ inline dim3 rc(int64_t rows, int64_t cols) { return ccl::rowcol_grid((int)rows, 
 inline dim3 rcb(const BatchTotals& t) { return ccl::rowcol_grid(t.rows, t.max_w); }
 inline dim3 qr(int64_t rows, int64_t cols) { return ccl::quadrow_grid((int)rows, (int)cols); }
 inline dim3 qrb(const BatchTotals& t) { return ccl::quadrow_grid(t.rows, t.max_w); }
+
+// Ranges that the labelling's first launch clears for a call: the status word, the bitmap, and
+// (optional) the counts.
+ccl::ZeroSpans call_spans(const Ws& w, bool bits, int counts) {
+  return ccl::ZeroSpans{{nullptr, (unsigned*)w.status, w.bits, (unsigned*)w.counts},
+                        {0, 1, bits ? (int)(w.bits_bytes / sizeof(unsigned)) : 0, counts}};
+}
 
 // Records the caller's optional timing event around the reconstruction kernel.  While the
 // stream is being captured into a CUDA graph the record becomes an external event-record node,
@@ -1120,16 +1135,21 @@ cudaError_t chain_impl(int dtype, const Plan& P, const Ws& w, int recon_conn, do
     });
     if (e == cudaSuccess)
       e = flood_launch(P.I, t.f_tiles, open, flooded, fill_conn, w.recon, s, opts ? opts->queue_poll_limit : 0);
-    if (e == cudaSuccess) e = ccl::label(ClsNotFlooded{flooded}, P.I, t, label_conn, w.forest(true), s);
+    if (e == cudaSuccess) {
+      // (the flooded plane lies in R, which the ranking overwrites after the labelling; the bitmap
+      // and the counts are cleared by the labelling's first launch)
+      ccl::ZeroSpans z = call_spans(w, true, 2 * t.n);
+      z.n[1] = 0;  // the status holds the reconstruction's
+      e = ccl::label(ClsNotFlooded{flooded}, P.I, t, label_conn, w.forest(true), s, z);
+    }
     if (e == cudaSuccess)
       e = ccl::rank_roots(P.I, t, w.forest(true), area_min, area_max, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre,
-                          w.counts, s);
-    if (e == cudaSuccess) {
-      label_out_kernel<true, true, true><<<qrb(t), 256, 0, s>>>(P.I, t.rows, w.L, w.R, labels_out, 0, w.A, area_min,
-                                                                area_max, nullptr, 0, area_out, 0, nullptr, fill_out,
-                                                                0);
-      e = cudaGetLastError();
-    }
+                          w.counts, s, nullptr, true, true);
+    if (e == cudaSuccess)
+      e = launch_dependent(label_out_kernel<true, true, true>, qrb(t), dim3(256), s, P.I, t.rows, (const int*)w.L,
+                           (const int*)w.R, labels_out, (int64_t)0, (const int*)w.A, area_min, area_max,
+                           (int32_t*)nullptr, (int64_t)0, area_out, (int64_t)0, (const unsigned*)nullptr, fill_out,
+                           (int64_t)0);
     return e;
   }
   if (e == cudaSuccess) {
@@ -1181,17 +1201,19 @@ cudaError_t candidates_impl(const Plan& P, const Ws& w, double g1, double g2, in
   unsigned* outside = (unsigned*)w.F;
   if (e == cudaSuccess)
     e = ccl::label_filled(ClsValleyAboveOrNot{gt1}, P.I, t, ccl::kConnFg8Bg4, w.forest(true), outside,
-                          w.bits_bytes, s, true);
-  if (e == cudaSuccess) e = ccl::count_roots(P.I, t, w.forest(true), lo, hi, w.bits, w.counts, s, outside);
-  if (e == cudaSuccess) e = cudaMemsetAsync(w.bits, 0, w.bits_bytes, s);
+                          w.bits_bytes, s, true, ccl::ZeroSpans{{nullptr, nullptr, (unsigned*)w.counts, nullptr}, {0, 0, 2 * t.n, 0}});
+  if (e == cudaSuccess)
+    e = ccl::count_roots(P.I, t, w.forest(true), lo, hi, w.bits, w.counts, s, outside, true);
   const ccl::Forest sel{w.R, nullptr, w.roots, w.nroots, nullptr};
-  if (e == cudaSuccess) e = ccl::label(ClsValleyAbove{gt2}, P.I, t, 8, sel, s);
-  if (e == cudaSuccess) {
-    ccl::ccl_seed_quads<SeedCandidate><<<qrb(t), 256, 0, s>>>(P.I, t.rows, w.R, SeedCandidate{gt2, w.L, w.A, lo, hi, outside},
-                                                               w.bits);
-    candidates_out_kernel<<<qrb(t), 256, 0, s>>>(P.I, t.rows, w.R, w.bits, rbc, out);
-    e = cudaGetLastError();
-  }
+  ccl::ZeroSpans z = call_spans(w, true, 0);
+  z.n[1] = 0;  // the status holds the reconstruction's
+  if (e == cudaSuccess) e = ccl::label(ClsValleyAbove{gt2}, P.I, t, 8, sel, s, z);
+  if (e == cudaSuccess)
+    e = launch_dependent(ccl::ccl_seed_quads<SeedCandidate>, qrb(t), dim3(256), s, P.I, t.rows, (const int*)w.R,
+                         SeedCandidate{gt2, w.L, w.A, lo, hi, outside}, w.bits);
+  if (e == cudaSuccess)
+    e = launch_dependent(candidates_out_kernel, qrb(t), dim3(256), s, P.I, t.rows, (const int*)w.R,
+                         (const unsigned*)w.bits, rbc, out);
   return e;
 }
 
@@ -1303,19 +1325,17 @@ nsgb_status nsgb_imreconstruct_binary(int dtype, void* marker, const void* mask,
   cudaStream_t s = (cudaStream_t)stream;
   const Plan P = single_plan(dtype, marker, mask, rows, cols, pitch);
   Ws w = carve(ws, P.t);
-  cudaError_t e = cudaMemsetAsync(w.status, 0, sizeof(int), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(w.bits, 0, w.bits_bytes, s);
-  if (e == cudaSuccess) {
-    e = dispatch_int(dtype, [&](auto* tag) -> cudaError_t {
-      using T = std::remove_pointer_t<decltype(tag)>;
-      ClsNonZero<T> cls{true};
-      cudaError_t r = ccl::label(cls, P.I, P.t, conn, w.forest(false), s);
-      if (r != cudaSuccess) return r;
-      ccl::ccl_seed_pixels<SeedBoth<T>><<<rc(rows, cols), 256, 0, s>>>(P.I, P.t.rows, w.L, SeedBoth<T>{true}, w.bits);
-      binrecon_out_kernel<T><<<rc(rows, cols), 256, 0, s>>>(P.I, P.t.rows, w.L, w.bits);
-      return cudaGetLastError();
-    });
-  }
+  cudaError_t e = dispatch_int(dtype, [&](auto* tag) -> cudaError_t {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    cudaError_t r = ccl::label(ClsNonZero<T>{true}, P.I, P.t, conn, w.forest(false), s, call_spans(w, true, 0));
+    if (r == cudaSuccess)
+      r = launch_dependent(ccl::ccl_seed_pixels<SeedBoth<T>>, rc(rows, cols), dim3(256), s, P.I, P.t.rows,
+                           (const int*)w.L, SeedBoth<T>{true}, w.bits);
+    if (r == cudaSuccess)
+      r = launch_dependent(binrecon_out_kernel<T>, rc(rows, cols), dim3(256), s, P.I, P.t.rows, (const int*)w.L,
+                           (const unsigned*)w.bits);
+    return r;
+  });
   return finish(e, ws, s, opts);
 }
 
@@ -1333,29 +1353,28 @@ nsgb_status nsgb_imfill_holes(int dtype, const void* image, void* out, int64_t r
   const int H = (int)rows, W = (int)cols;
   const Plan P = single_plan(dtype, (void*)image, nullptr, rows, cols, pitch);
   Ws w = carve(ws, P.t);
-  cudaError_t e = cudaMemsetAsync(w.status, 0, sizeof(int), s);
-  if (e != cudaSuccess) return NSGB_ERR_CUDA;
+  cudaError_t e = cudaSuccess;
   if (binary) {
     if (dtype == NSGB_I32) {
       // min<int> is non-zero, so the reference's binary reconstruction has no background to
       // grow into and every pixel comes back as invert(min<int>) = INT_MAX.
+      e = cudaMemsetAsync(w.status, 0, sizeof(int), s);
+      if (e != cudaSuccess) return NSGB_ERR_CUDA;
       fill_const_kernel<int32_t><<<rc(rows, cols), 256, 0, s>>>((int32_t*)out, pitch, H, W, INT_MAX);
       return finish(cudaGetLastError(), ws, s, opts);
     }
-    e = cudaMemsetAsync(w.bits, 0, w.bits_bytes, s);
-    if (e == cudaSuccess) {
-      e = dispatch_int(dtype, [&](auto* tag) -> cudaError_t {
-        using T = std::remove_pointer_t<decltype(tag)>;
-        ClsNotMax<T> cls;
-        cudaError_t r = ccl::label(cls, P.I, P.t, conn, w.forest(false), s);
-        if (r != cudaSuccess) return r;
-        ccl::ccl_seed_border<SeedBorder<ClsNotMax<T>>><<<dim3(grid1d(2 * (rows + cols)), 1), 256, 0, s>>>(
-            P.I, w.L, SeedBorder<ClsNotMax<T>>{cls}, w.bits);
-        fill_out_kernel<T><<<qr(rows, cols), 256, 0, s>>>(P.I, P.t.rows, w.L, w.bits, nullptr, (T*)out, pitch,
-                                                          std::numeric_limits<T>::max());
-        return cudaGetLastError();
-      });
-    }
+    e = dispatch_int(dtype, [&](auto* tag) -> cudaError_t {
+      using T = std::remove_pointer_t<decltype(tag)>;
+      ClsNotMax<T> cls;
+      cudaError_t r = ccl::label(cls, P.I, P.t, conn, w.forest(false), s, call_spans(w, true, 0));
+      if (r == cudaSuccess)
+        r = launch_dependent(ccl::ccl_seed_border<SeedBorder<ClsNotMax<T>>>, dim3(grid1d(2 * (rows + cols)), 1),
+                             dim3(256), s, P.I, (const int*)w.L, SeedBorder<ClsNotMax<T>>{cls}, w.bits);
+      if (r == cudaSuccess)
+        r = launch_dependent(fill_out_kernel<T>, qr(rows, cols), dim3(256), s, P.I, P.t.rows, (const int*)w.L,
+                             (const unsigned*)w.bits, (uint8_t*)nullptr, (T*)out, pitch, std::numeric_limits<T>::max());
+      return r;
+    });
     return finish(e, ws, s, opts);
   }
   // Grayscale: erosion reconstruction of (image on the border, max inside) above the image.
@@ -1417,21 +1436,18 @@ nsgb_status nsgb_bwselect(int dtype, const void* image, const void* seeds, void*
   cudaStream_t s = (cudaStream_t)stream;
   const Plan P = single_plan(dtype, (void*)image, seeds, rows, cols, pitch);
   Ws w = carve(ws, P.t);
-  cudaError_t e = cudaMemsetAsync(w.status, 0, sizeof(int), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(w.bits, 0, w.bits_bytes, s);
-  if (e == cudaSuccess) {
-    e = dispatch_int(dtype, [&](auto* tag) -> cudaError_t {
-      using T = std::remove_pointer_t<decltype(tag)>;
-      ClsNonZero<T> cls{false};
-      cudaError_t r = ccl::label(cls, P.I, P.t, conn, w.forest(false), s);
-      if (r != cudaSuccess) return r;
-      // seeds (aux) != 0 and image (plane) != 0
-      ccl::ccl_seed_pixels<SeedBoth<T>><<<rc(rows, cols), 256, 0, s>>>(P.I, P.t.rows, w.L, SeedBoth<T>{false},
-                                                                        w.bits);
-      bwselect_out_kernel<T><<<rc(rows, cols), 256, 0, s>>>(P.I, P.t.rows, out, w.L, w.bits);
-      return cudaGetLastError();
-    });
-  }
+  cudaError_t e = dispatch_int(dtype, [&](auto* tag) -> cudaError_t {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    cudaError_t r = ccl::label(ClsNonZero<T>{false}, P.I, P.t, conn, w.forest(false), s, call_spans(w, true, 0));
+    // seeds (aux) != 0 and image (plane) != 0
+    if (r == cudaSuccess)
+      r = launch_dependent(ccl::ccl_seed_pixels<SeedBoth<T>>, rc(rows, cols), dim3(256), s, P.I, P.t.rows,
+                           (const int*)w.L, SeedBoth<T>{false}, w.bits);
+    if (r == cudaSuccess)
+      r = launch_dependent(bwselect_out_kernel<T>, rc(rows, cols), dim3(256), s, P.I, P.t.rows, out, (const int*)w.L,
+                           (const unsigned*)w.bits);
+    return r;
+  });
   return finish(e, ws, s, opts);
 }
 
@@ -1446,19 +1462,15 @@ nsgb_status nsgb_bwlabel(const uint8_t* bin, int32_t* labels, int64_t rows, int6
   cudaStream_t s = (cudaStream_t)stream;
   const Plan P = single_plan(NSGB_U8, (void*)bin, nullptr, rows, cols, pitch_in);
   Ws w = carve(ws, P.t);
-  cudaError_t e = cudaMemsetAsync(w.status, 0, sizeof(int), s);
-  if (e != cudaSuccess) return NSGB_ERR_CUDA;
-  e = ccl::label(ClsValueU8{}, P.I, P.t, conn, w.forest(false), s);
-  if (e == cudaSuccess) e = ccl::rank_roots(P.I, P.t, w.forest(false), 0, 0, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre, w.counts, s);
-  if (e == cudaSuccess) {
-    if (relabel)
-      label_out_kernel<true, false><<<qr(rows, cols), 256, 0, s>>>(P.I, P.t.rows, w.L, w.R, labels, pitch_labels,
-                                                                   nullptr, 0, 0, nullptr, 0, nullptr, 0);
-    else
-      label_out_kernel<false, false><<<qr(rows, cols), 256, 0, s>>>(P.I, P.t.rows, w.L, w.R, labels, pitch_labels,
-                                                                    nullptr, 0, 0, nullptr, 0, nullptr, 0);
-    e = cudaGetLastError();
-  }
+  cudaError_t e = ccl::label(ClsValueU8{}, P.I, P.t, conn, w.forest(false), s, call_spans(w, true, 2));
+  if (e == cudaSuccess)
+    e = ccl::rank_roots(P.I, P.t, w.forest(false), 0, 0, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre, w.counts, s, nullptr,
+                        true, true);
+  if (e == cudaSuccess)
+    e = launch_dependent(relabel ? label_out_kernel<true, false> : label_out_kernel<false, false>, qr(rows, cols),
+                         dim3(256), s, P.I, P.t.rows, (const int*)w.L, (const int*)w.R, labels, pitch_labels,
+                         (const int*)nullptr, 0, 0, (int32_t*)nullptr, (int64_t)0, (uint8_t*)nullptr, (int64_t)0,
+                         (const unsigned*)nullptr, (uint8_t*)nullptr, (int64_t)0);
   if (e == cudaSuccess && count) {
     e = cudaMemcpyAsync(count, w.counts, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1480,24 +1492,24 @@ nsgb_status nsgb_bwareaopen(const void* in, int labeled, int32_t* labels_out, ui
   const int64_t n = rows * cols;
   const Plan P = single_plan(NSGB_U8, (void*)in, nullptr, rows, cols, pitch_in);
   Ws w = carve(ws, P.t);
-  cudaError_t e = cudaMemsetAsync(w.status, 0, sizeof(int), s);
-  if (e != cudaSuccess) return NSGB_ERR_CUDA;
+  cudaError_t e = cudaSuccess;
   if (!labeled) {
-    e = ccl::label(ClsValueU8{}, P.I, P.t, conn, w.forest(true), s);
-    if (e == cudaSuccess) e = ccl::rank_roots(P.I, P.t, w.forest(true), min_size, max_size, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre, w.counts, s);
-    if (e == cudaSuccess) {
-      label_out_kernel<false, true><<<qr(rows, cols), 256, 0, s>>>(P.I, P.t.rows, w.L, w.R, nullptr, 0, w.A, min_size,
-                                                                   max_size, labels_out, pitch_labels, flat_out,
-                                                                   pitch_flat);
-      e = cudaGetLastError();
-    }
+    e = ccl::label(ClsValueU8{}, P.I, P.t, conn, w.forest(true), s, call_spans(w, true, 2));
+    if (e == cudaSuccess)
+      e = ccl::rank_roots(P.I, P.t, w.forest(true), min_size, max_size, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre, w.counts,
+                          s, nullptr, true, true);
+    if (e == cudaSuccess)
+      e = launch_dependent(label_out_kernel<false, true>, qr(rows, cols), dim3(256), s, P.I, P.t.rows, (const int*)w.L,
+                           (const int*)w.R, (int32_t*)nullptr, (int64_t)0, (const int*)w.A, min_size, max_size, labels_out,
+                           pitch_labels, flat_out, pitch_flat, (const unsigned*)nullptr, (uint8_t*)nullptr, (int64_t)0);
     if (e == cudaSuccess && count) {
       e = cudaMemcpyAsync(count, w.counts + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
     return finish(e, ws, s, opts);
   }
-  e = cudaMemsetAsync(w.A, 0, sizeof(int) * (size_t)n, s);
+  e = cudaMemsetAsync(w.status, 0, sizeof(int), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(w.A, 0, sizeof(int) * (size_t)n, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(w.counts, 0, 2 * sizeof(int), s);
   if (e == cudaSuccess) {
     label_hist_kernel<<<rc(rows, cols), 256, 0, s>>>(P.I, P.t.rows, w.A, w.status);
