@@ -693,7 +693,6 @@ Ws carve(void* ws, const BatchTotals& t) {
 
 inline int grid1d(int64_t n) { return ccl::flat_grid(n); }
 inline dim3 rc(int64_t rows, int64_t cols) { return ccl::rowcol_grid((int)rows, (int)cols); }
-inline dim3 rcb(const BatchTotals& t) { return ccl::rowcol_grid(t.rows, t.max_w); }
 inline dim3 qr(int64_t rows, int64_t cols) { return ccl::quadrow_grid((int)rows, (int)cols); }
 inline dim3 qrb(const BatchTotals& t) { return ccl::quadrow_grid(t.rows, t.max_w); }
 
@@ -1217,6 +1216,16 @@ cudaError_t candidates_impl(const Plan& P, const Ws& w, double g1, double g2, in
   return e;
 }
 
+// The image of every reconstruction tile and of every labelling tile: blockIdx.y walks the images.
+__global__ void batch_maps_kernel(const Img* __restrict__ table, int n, int* __restrict__ r_img, int* __restrict__ c_img) {
+  for (int i = blockIdx.y; i < n; i += gridDim.y) {
+    const Img& m = table[i];
+    const int nr = m.r_tiles_x * m.r_tiles_y, nc = m.c_tiles_x * ((m.H + ccl::kTile - 1) / ccl::kTile);
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nr; k += gridDim.x * blockDim.x) r_img[m.r_tile_base + k] = i;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nc; k += gridDim.x * blockDim.x) c_img[m.c_tile_base + k] = i;
+  }
+}
+
 }  // namespace
 }  // namespace nsgb
 
@@ -1230,18 +1239,32 @@ bool want_sync(const nsgb_opts* o) { return o == nullptr || o->sync != 0; }
 
 nsgb_status cuda_status(cudaError_t e) { return e == cudaSuccess ? NSGB_OK : NSGB_ERR_CUDA; }
 
-// Finishes a call: reports launch errors; with sync, waits and reports the device status.
-nsgb_status finish(cudaError_t e, const void* ws, cudaStream_t s, const nsgb_opts* o) {
+// Finishes a call: reports launch errors; with sync, waits and reports the device status.  With
+// `n` > 0 the counts (n words of the workspace, which may start with the status) are read too, sync or not.  Status
+// and counts come in one strided copy where the distance allows it: each copy to pageable memory
+// is a round trip of its own (about 8 us).
+nsgb_status finish(cudaError_t e, const void* ws, cudaStream_t s, const nsgb_opts* o, const int* counts = nullptr,
+                   int n = 0, int32_t* to = nullptr) {
   if (e != cudaSuccess) return NSGB_ERR_CUDA;
   e = cudaGetLastError();
   if (e != cudaSuccess) return NSGB_ERR_CUDA;
-  if (!want_sync(o)) return NSGB_OK;
-  int dev_status = 0;
-  e = cudaMemcpyAsync(&dev_status, ws, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (n == 0 && !want_sync(o)) return NSGB_OK;
+  constexpr int kRow = 32;
+  const int64_t apart = n > 0 ? (const char*)counts - (const char*)ws : 0;
+  int32_t both[2][kRow] = {};
+  if (n > 0 && n <= kRow && apart >= (int64_t)sizeof(int) * kRow && apart < (int64_t)INT_MAX) {
+    e = cudaMemcpy2DAsync(both, sizeof(both[0]), ws, (size_t)apart, sizeof(int) * (size_t)n, 2, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) memcpy(to, both[1], sizeof(int) * (size_t)n);
+  } else {
+    if (n > 0) e = cudaMemcpyAsync(to, counts, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && (n == 0 || apart != 0))
+      e = cudaMemcpyAsync(&both[0][0], ws, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (n > 0 && apart == 0) both[0][0] = to[0];
+  }
   if (e != cudaSuccess) return NSGB_ERR_CUDA;
-  e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return NSGB_ERR_CUDA;
-  return (nsgb_status)dev_status;
+  return want_sync(o) ? (nsgb_status)both[0][0] : NSGB_OK;
 }
 
 nsgb_status check_ws_bytes(void* ws, size_t ws_bytes, size_t need) {
@@ -1471,11 +1494,7 @@ nsgb_status nsgb_bwlabel(const uint8_t* bin, int32_t* labels, int64_t rows, int6
                          dim3(256), s, P.I, P.t.rows, (const int*)w.L, (const int*)w.R, labels, pitch_labels,
                          (const int*)nullptr, 0, 0, (int32_t*)nullptr, (int64_t)0, (uint8_t*)nullptr, (int64_t)0,
                          (const unsigned*)nullptr, (uint8_t*)nullptr, (int64_t)0);
-  if (e == cudaSuccess && count) {
-    e = cudaMemcpyAsync(count, w.counts, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  }
-  return finish(e, ws, s, opts);
+  return finish(e, ws, s, opts, w.counts, count ? 1 : 0, count);
 }
 
 nsgb_status nsgb_bwareaopen(const void* in, int labeled, int32_t* labels_out, uint8_t* flat_out, int64_t rows,
@@ -1502,11 +1521,7 @@ nsgb_status nsgb_bwareaopen(const void* in, int labeled, int32_t* labels_out, ui
       e = launch_dependent(label_out_kernel<false, true>, qr(rows, cols), dim3(256), s, P.I, P.t.rows, (const int*)w.L,
                            (const int*)w.R, (int32_t*)nullptr, (int64_t)0, (const int*)w.A, min_size, max_size, labels_out,
                            pitch_labels, flat_out, pitch_flat, (const unsigned*)nullptr, (uint8_t*)nullptr, (int64_t)0);
-    if (e == cudaSuccess && count) {
-      e = cudaMemcpyAsync(count, w.counts + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    }
-    return finish(e, ws, s, opts);
+    return finish(e, ws, s, opts, w.counts + 1, count ? 1 : 0, count);
   }
   e = cudaMemsetAsync(w.status, 0, sizeof(int), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(w.A, 0, sizeof(int) * (size_t)n, s);
@@ -1518,11 +1533,7 @@ nsgb_status nsgb_bwareaopen(const void* in, int labeled, int32_t* labels_out, ui
                                                             pitch_labels, flat_out, pitch_flat);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess && count) {
-    e = cudaMemcpyAsync(count, w.counts + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  }
-  return finish(e, ws, s, opts);
+  return finish(e, ws, s, opts, w.counts + 1, count ? 1 : 0, count);
 }
 
 nsgb_status nsgb_bounding_boxes(const int32_t* labels, int64_t rows, int64_t cols, int64_t pitch, int32_t bgval,
@@ -1535,11 +1546,11 @@ nsgb_status nsgb_bounding_boxes(const int32_t* labels, int64_t rows, int64_t col
   cudaStream_t s = (cudaStream_t)stream;
   const Plan P = single_plan(NSGB_I32, (void*)labels, nullptr, rows, cols, pitch);
   cudaError_t e = bbox_launch(P.I, P.t, bgval, ws, boxes, capacity, count_dev, s);
-  if (e == cudaSuccess && count) {
-    e = cudaMemcpyAsync(count, (const int*)ws + 2, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  }
-  return finish(e, ws, s, opts);
+  // the count sits in the header, two words behind the status
+  int32_t head[3] = {};
+  const nsgb_status r = finish(e, ws, s, opts, (const int*)ws, count ? 3 : 0, head);
+  if (count && r != NSGB_ERR_CUDA) *count = head[2];
+  return r;
 }
 
 nsgb_status nsgb_morph_open(const uint8_t* in, uint8_t* out, int64_t rows, int64_t cols, int64_t pitch_in,
@@ -1589,11 +1600,7 @@ nsgb_status nsgb_nucleus_candidates(uint8_t* rc_open, const uint8_t* rc, const u
   cudaError_t e = candidates_impl(P, w, g1, g2, area_min, area_max, rbc, seg_out, opts, s);
   if (e == cudaSuccess && n_kept_dev)
     e = cudaMemcpyAsync(n_kept_dev, w.counts + 1, sizeof(int32_t), cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess && n_kept) {
-    e = cudaMemcpyAsync(n_kept, w.counts + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  }
-  return finish(e, ws, s, opts);
+  return finish(e, ws, s, opts, w.counts + 1, n_kept ? 1 : 0, n_kept);
 }
 
 nsgb_status nsgb_threshold(int dtype, const void* in, uint8_t* out, int64_t rows, int64_t cols, int64_t pitch_in,
@@ -1647,14 +1654,13 @@ nsgb_status nsgb_chain(int dtype, void* marker, const void* mask, int64_t rows, 
   Ws w = carve(ws, P.t);
   cudaError_t e = chain_impl(dtype, P, w, recon_conn, thr, fill_conn, label_conn, area_min, area_max, fill_out,
                              labels_out, area_out, opts, s);
-  if (e == cudaSuccess && (n_labels || n_kept)) {
-    int32_t c[2] = {0, 0};
-    e = cudaMemcpyAsync(c, w.counts, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  int32_t c[2] = {0, 0};
+  const nsgb_status r = finish(e, ws, s, opts, w.counts, n_labels || n_kept ? 2 : 0, c);
+  if (r != NSGB_ERR_CUDA) {
     if (n_labels) *n_labels = c[0];
     if (n_kept) *n_kept = c[1];
   }
-  return finish(e, ws, s, opts);
+  return r;
 }
 
 }  // extern "C"
@@ -1736,20 +1742,12 @@ nsgb_status nsgb_batch_prepare(int dtype, const nsgb_tile* tiles, int n_tiles, v
   nsgb_status st = check_ws_bytes(ws, ws_bytes, nsgb_batch_workspace_size(dtype, tiles, n_tiles));
   if (st != NSGB_OK) return st;
   Ws w = carve(ws, table_totals(t));
-  // The tile maps: image of every reconstruction tile, then of every labelling tile.
-  std::vector<int> maps((size_t)t.r_tiles + (size_t)t.c_tiles);
-  for (int i = 0; i < (int)imgs.size(); ++i) {
-    const Img& m = imgs[i];
-    const int nr = m.r_tiles_x * m.r_tiles_y;
-    const int nc = m.c_tiles_x * ((m.H + ccl::kTile - 1) / ccl::kTile);
-    std::fill(maps.begin() + m.r_tile_base, maps.begin() + m.r_tile_base + nr, i);
-    std::fill(maps.begin() + t.r_tiles + m.c_tile_base, maps.begin() + t.r_tiles + m.c_tile_base + nc, i);
-  }
-  // Synchronous copies: the host arrays go away when this returns.
+  // Synchronous copy: the host array goes away when this returns.  The tile maps (image of every
+  // reconstruction tile, then of every labelling tile) are written on the device from the table.
   if (cudaMemcpy(w.table, imgs.data(), sizeof(Img) * imgs.size(), cudaMemcpyHostToDevice) != cudaSuccess)
     return NSGB_ERR_CUDA;
-  if (cudaMemcpy(w.r_img, maps.data(), sizeof(int) * maps.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-    return NSGB_ERR_CUDA;
+  batch_maps_kernel<<<dim3(8, (unsigned)std::min(t.n, 65535)), 256>>>(w.table, t.n, w.r_img, w.c_img);
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) return NSGB_ERR_CUDA;
   memset(batch, 0, sizeof(*batch));
   batch->dtype = dtype;
   batch->n = t.n;
@@ -1779,16 +1777,13 @@ nsgb_status nsgb_chain_batch(const nsgb_batch* batch, int recon_conn, double thr
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = chain_impl(batch->dtype, P, w, recon_conn, thr, fill_conn, label_conn, area_min, area_max,
                              nullptr, nullptr, nullptr, opts, s);
-  if (e == cudaSuccess && (n_labels || n_kept)) {
-    std::vector<int32_t> c(2 * (size_t)P.t.n);
-    e = cudaMemcpyAsync(c.data(), w.counts, c.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    for (int i = 0; i < P.t.n && e == cudaSuccess; ++i) {
-      if (n_labels) n_labels[i] = c[2 * i];
-      if (n_kept) n_kept[i] = c[2 * i + 1];
-    }
+  std::vector<int32_t> c(n_labels || n_kept ? 2 * (size_t)P.t.n : 0);
+  const nsgb_status r = finish(e, w.status, s, opts, w.counts, (int)c.size(), c.data());
+  for (int i = 0; i < P.t.n && r != NSGB_ERR_CUDA; ++i) {
+    if (n_labels) n_labels[i] = c[2 * i];
+    if (n_kept) n_kept[i] = c[2 * i + 1];
   }
-  return finish(e, w.status, s, opts);
+  return r;
 }
 
 nsgb_status nsgb_batch_counts_async(const nsgb_batch* batch, int32_t* counts, nsgb_stream_t stream) {

@@ -14,6 +14,7 @@ C ABI directly (opts.sync = 0).
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -51,8 +52,8 @@ def _pitch(t: torch.Tensor) -> int:
     return t.stride(0) * t.element_size()
 
 
-def _stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    return torch.cuda.current_stream().cuda_stream
 
 
 class _Workspace:
@@ -75,9 +76,11 @@ class _Workspace:
 workspace = _Workspace()
 
 
+_workspace_size = functools.lru_cache(maxsize=256)(lib.nsgb_workspace_size)
+
+
 def _ws(op: int, dtype: int, rows: int, cols: int, device: torch.device) -> Tuple[int, int]:
-    need = lib.nsgb_workspace_size(op, dtype, rows, cols)
-    return workspace.get(need, device)
+    return workspace.get(_workspace_size(op, dtype, rows, cols), device)
 
 
 def _same_shape(a: torch.Tensor, b: torch.Tensor, what: str) -> None:
@@ -412,21 +415,24 @@ class BatchPlan:
         self.masks = [_contig(m) for m in masks]
         self.fill, self.labels, self.area = [], [], []
         tiles = (_ffi.Tile * len(markers))()
-        for i, (mk, ms) in enumerate(zip(self.markers, self.masks)):
+        for tile, mk, ms in zip(tiles, self.markers, self.masks):
             _check_image(mk, "marker")
             _check_image(ms, "mask")
             _same_shape(mk, ms, "batch")
             if _dtype_code(ms) != dt:
                 raise NsgbError(1, "batch: all tiles must share one dtype")
-            rows, cols = ms.shape
+            shape, dev = ms.shape, ms.device
+            tile.marker, tile.mask = mk.data_ptr(), ms.data_ptr()
+            tile.rows, tile.cols = shape
+            tile.pitch = _pitch(ms)
             if with_outputs:
-                self.fill.append(torch.empty((rows, cols), dtype=torch.uint8, device=ms.device))
-                self.labels.append(torch.empty((rows, cols), dtype=torch.int32, device=ms.device))
-                self.area.append(torch.empty((rows, cols), dtype=torch.uint8, device=ms.device))
-            tiles[i] = _ffi.Tile(mk.data_ptr(), ms.data_ptr(), rows, cols, _pitch(ms),
-                                 self.fill[i].data_ptr() if with_outputs else None,
-                                 self.labels[i].data_ptr() if with_outputs else None,
-                                 self.area[i].data_ptr() if with_outputs else None)
+                fill = torch.empty(shape, dtype=torch.uint8, device=dev)
+                labels = torch.empty(shape, dtype=torch.int32, device=dev)
+                area = torch.empty(shape, dtype=torch.uint8, device=dev)
+                self.fill.append(fill)
+                self.labels.append(labels)
+                self.area.append(area)
+                tile.fill_out, tile.labels_out, tile.area_out = fill.data_ptr(), labels.data_ptr(), area.data_ptr()
         need = lib.nsgb_batch_workspace_size(dt, tiles, len(markers))
         if need == 0:
             raise NsgbError(1, "batch: bad tiles (or more than 2^31 pixels in total)")
