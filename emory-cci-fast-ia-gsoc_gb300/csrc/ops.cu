@@ -339,12 +339,49 @@ __global__ void candidates_out_kernel(Imgs I, int total_rows, const int* __restr
 
 // Labels out: relabel ? (bg 0, root's rank + 1) : the root's raster index in its image / -1.
 // Optional area-filter outputs from the same pass.  rank / A are read-only here: L1-cached
-// loads, because a giant component's root is read by every one of its pixels.  Single image:
-// explicit output pointers / pitches; batch: Img::labels / Img::area (dense).
+// loads, because a giant component's root is read by every one of its pixels.
 // RELABEL: raster rank labels (else root indices); AREA: area-filter outputs (A non-null).
-// FILLED: the labelled pixels are the filled image, written as 255 (0 elsewhere) to `filled`
-// (single image, optional) or Img::fill (batch); with `outside` (the forest of
-// ccl::label_filled) the roots it marks are background too.
+// FILLED: the labelled pixels are the filled image (255, 0 elsewhere); with `outside` (the forest
+// of ccl::label_filled) the roots it marks are background too.
+struct LabelQuad {
+  int lab[4], kept[4];
+  uint8_t flat[4], filled[4];
+};
+template <bool RELABEL, bool AREA, bool FILLED>
+__device__ __forceinline__ void label_quad(int (&r)[4], int px_base, const int* __restrict__ rank,
+                                           const int* __restrict__ A, int lo, int hi,
+                                           const unsigned* __restrict__ outside, LabelQuad& q) {
+  if (FILLED) {
+    bool out[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      out[k] = (k > 0 && r[k] == r[k - 1]) ? out[k - 1] : (r[k] >= 0 && outside && ccl::test_bit(outside, r[k]));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (out[k]) r[k] = -1;
+      q.filled[k] = r[k] >= 0 ? 255 : 0;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const bool same = k > 0 && r[k] == r[k - 1];
+    q.lab[k] = same ? q.lab[k - 1]
+                    : (RELABEL ? (r[k] < 0 ? 0 : __ldg(&rank[r[k]]) + 1) : (r[k] < 0 ? -1 : r[k] - px_base));
+    bool keep = false;
+    if (AREA) {
+      if (same) {
+        keep = q.flat[k - 1] != 0;
+      } else {
+        const int a = r[k] >= 0 ? __ldg(&A[r[k]]) : 0;
+        keep = r[k] >= 0 && a >= lo && a < hi;
+      }
+    }
+    q.flat[k] = keep ? 255 : 0;
+    q.kept[k] = keep ? r[k] - px_base : -1;
+  }
+}
+
+// Single image: explicit output pointers / pitches (`filled` optional); a table of one: Img's.
 template <bool RELABEL, bool AREA, bool FILLED = false>
 __global__ void label_out_kernel(Imgs I, int total_rows, const int* __restrict__ L, const int* __restrict__ rank,
                                  int32_t* labels, int64_t pitch_labels, const int* __restrict__ A, int lo,
@@ -354,53 +391,54 @@ __global__ void label_out_kernel(Imgs I, int total_rows, const int* __restrict__
   pdl_wait();
   pdl_release();
   ccl::for_batch_quads(I, total_rows, [&](const Img& m, int y, int x, int n) {
-    int r[4], lab[4], kl[4];
-    uint8_t fl[4];
+    int r[4];
+    LabelQuad q;
     ccl::roots4_ro(L, (int64_t)m.px_base + (int64_t)y * m.W + x, n, r);
-    if (FILLED) {
-      bool out[4];
-      uint8_t fi[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        out[k] = (k > 0 && r[k] == r[k - 1]) ? out[k - 1] : (r[k] >= 0 && outside && ccl::test_bit(outside, r[k]));
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (out[k]) r[k] = -1;
-        fi[k] = r[k] >= 0 ? 255 : 0;
-      }
-      if (!I.d) {
-        if (filled) store4_u8(pxp<uint8_t>(filled, pitch_filled, y, x), n, fi);
-      } else if (m.fill) {
-        store4_u8(m.fill + (int64_t)y * m.W + x, n, fi);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const bool same = k > 0 && r[k] == r[k - 1];
-      lab[k] = same ? lab[k - 1]
-                    : (RELABEL ? (r[k] < 0 ? 0 : __ldg(&rank[r[k]]) + 1) : (r[k] < 0 ? -1 : r[k] - m.px_base));
-      bool keep = false;
-      if (AREA) {
-        if (same) {
-          keep = fl[k - 1] != 0;
-        } else {
-          const int a = r[k] >= 0 ? __ldg(&A[r[k]]) : 0;
-          keep = r[k] >= 0 && a >= lo && a < hi;
-        }
-      }
-      fl[k] = keep ? 255 : 0;
-      kl[k] = keep ? r[k] - m.px_base : -1;
-    }
+    label_quad<RELABEL, AREA, FILLED>(r, m.px_base, rank, A, lo, hi, outside, q);
     if (!I.d) {
-      if (labels) store4_i32(pxp<int32_t>(labels, pitch_labels, y, x), n, lab);
-      if (AREA && kept_labels) store4_i32(pxp<int32_t>(kept_labels, pitch_kept, y, x), n, kl);
-      if (AREA && flat) store4_u8(pxp<uint8_t>(flat, pitch_flat, y, x), n, fl);
+      if (FILLED && filled) store4_u8(pxp<uint8_t>(filled, pitch_filled, y, x), n, q.filled);
+      if (labels) store4_i32(pxp<int32_t>(labels, pitch_labels, y, x), n, q.lab);
+      if (AREA && kept_labels) store4_i32(pxp<int32_t>(kept_labels, pitch_kept, y, x), n, q.kept);
+      if (AREA && flat) store4_u8(pxp<uint8_t>(flat, pitch_flat, y, x), n, q.flat);
     } else {
       const int64_t li = (int64_t)y * m.W + x;
-      if (m.labels) store4_i32(m.labels + li, n, lab);
-      if (AREA && m.area) store4_u8(m.area + li, n, fl);
+      if (FILLED && m.fill) store4_u8(m.fill + li, n, q.filled);
+      if (m.labels) store4_i32(m.labels + li, n, q.lab);
+      if (AREA && m.area) store4_u8(m.area + li, n, q.flat);
     }
   });
+}
+
+// The same for a batch, whose outputs are dense: an image is a line of pixels, and every quad of
+// it is aligned in the label plane (px_base is a multiple of 4) and in outputs that start aligned,
+// whatever the width -- row by row an odd width left three rows of four to scalar accesses (71
+// Mpixel of uneven u8 tiles: 211 us row by row, 99 us along the line).  A CTA takes kLineBlocks
+// consecutive rank blocks of 1024 pixels and looks its image up once.
+constexpr int kLineBlocks = 4;
+template <bool RELABEL, bool AREA, bool FILLED>
+__global__ void __launch_bounds__(ccl::kBlockPx / 4) label_line_kernel(Imgs I, int nblocks, const int* __restrict__ L,
+                                                                       const int* __restrict__ rank,
+                                                                       const int* __restrict__ A, int lo, int hi) {
+  pdl_wait();
+  pdl_release();
+  const int b0 = blockIdx.x * kLineBlocks, b1 = min(nblocks, b0 + kLineBlocks);
+  int ii = img_of(I, b0, BlkBase());
+  for (int b = b0; b < b1; ++b) {
+    while (ii + 1 < I.n && b >= I.d[ii + 1].blk_base) ++ii;
+    const Img& m = I.d[ii];
+    const int px_base = m.px_base;
+    const int64_t at = (int64_t)(b - m.blk_base) * ccl::kBlockPx + 4 * threadIdx.x;
+    const int64_t left = (int64_t)m.H * m.W - at;
+    if (left <= 0) continue;
+    const int n = (int)min((int64_t)4, left);
+    int r[4];
+    LabelQuad q;
+    ccl::roots4_ro(L, px_base + at, n, r);
+    label_quad<RELABEL, AREA, FILLED>(r, px_base, rank, A, lo, hi, nullptr, q);
+    if (FILLED && m.fill) store4_u8(m.fill + at, n, q.filled);
+    if (m.labels) store4_i32(m.labels + at, n, q.lab);
+    if (AREA && m.area) store4_u8(m.area + at, n, q.flat);
+  }
 }
 
 // Area of arbitrary int32 labels in [-1, n): dense histogram (background -1 skipped).
@@ -587,6 +625,7 @@ void add_image(Img& m, BatchTotals& t) {
   m.r_even_base = t.r_even;
   for (int c = 0; c < 3; ++c) m.r_col_base[c] = t.r_col[c];
   m.c_tile_base = t.c_tiles;
+  t.px = (t.px + 3) & ~(int64_t)3;  // four pixels of an image's label plane are one aligned load
   m.px_base = (int)t.px;
   m.blk_base = t.blocks;
   m.row_base = t.rows;
@@ -1145,10 +1184,9 @@ cudaError_t chain_impl(int dtype, const Plan& P, const Ws& w, int recon_conn, do
       e = ccl::rank_roots(P.I, t, w.forest(true), area_min, area_max, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre,
                           w.counts, s, nullptr, true, true);
     if (e == cudaSuccess)
-      e = launch_dependent(label_out_kernel<true, true, true>, qrb(t), dim3(256), s, P.I, t.rows, (const int*)w.L,
-                           (const int*)w.R, labels_out, (int64_t)0, (const int*)w.A, area_min, area_max,
-                           (int32_t*)nullptr, (int64_t)0, area_out, (int64_t)0, (const unsigned*)nullptr, fill_out,
-                           (int64_t)0);
+      e = launch_dependent(label_line_kernel<true, true, true>, dim3((t.blocks + kLineBlocks - 1) / kLineBlocks),
+                           dim3(ccl::kBlockPx / 4), s, P.I, t.blocks, (const int*)w.L, (const int*)w.R,
+                           (const int*)w.A, area_min, area_max);
     return e;
   }
   if (e == cudaSuccess) {
