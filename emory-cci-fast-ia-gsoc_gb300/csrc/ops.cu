@@ -169,21 +169,59 @@ struct SeedBoth {  // a != 0 and b != 0, with a = plane or aux as selected
 };
 
 // bwselect's seeds in the nucleus-candidate stage: D > g2 on a pixel of a filled component
-// (forest LF, areas A) whose area lies in [lo, hi) -- bw2 & bw1_t without writing bw1_t.
-struct SeedCandidate {
+// (forest LF, areas A) whose area lies in [lo, hi) -- bw2 & bw1_t without writing bw1_t.  A seed
+// marks its root in the forest L2 of D > g2.  Four pixels per thread; rc and R come as one 32-bit
+// load each where rows allow it (`words`), and few quads hold a pixel above g2 (byte loads and
+// the filled component's lookups one pixel after another took 69 us at 4096^2, this 49).
+struct CandidateSeeds {
   GtThr<uint8_t> gt;
   const int* LF;
   const int* A;
   int lo, hi;
-  const unsigned* outside;  // roots of LF that are not part of the filled image (optional)
-  __device__ bool operator()(const Img& m, int y, int x) const {
-    if (!gt(valley(m, y, x))) return false;
-    const int r = ccl::root_of_ro(LF, (int64_t)m.px_base + (int64_t)y * m.W + x);
-    if (r < 0 || (outside && ccl::test_bit(outside, r))) return false;
-    const int a = __ldg(A + r);
-    return a >= lo && a < hi;
-  }
+  const unsigned* outside;  // roots of LF that are not part of the filled image
+  bool words;
 };
+__global__ void candidate_seeds_kernel(Imgs I, int total_rows, const int* __restrict__ L2, CandidateSeeds c,
+                                       unsigned* __restrict__ bits) {
+  pdl_wait();
+  pdl_release();
+  ccl::for_batch_quads(I, total_rows, [&](const Img& m, int y, int x, int n) {
+    const uint8_t* rc = (const uint8_t*)m.aux + (int64_t)y * m.pitch + x;
+    const uint8_t* rec = (const uint8_t*)m.plane + (int64_t)y * m.pitch + x;
+    uint32_t a = 0, b = 0;
+    if (c.words && n == 4) {
+      a = *(const uint32_t*)rc;
+      b = *(const uint32_t*)rec;
+    } else {
+      for (int k = 0; k < n; ++k) {
+        a |= (uint32_t)rc[k] << (8 * k);
+        b |= (uint32_t)rec[k] << (8 * k);
+      }
+    }
+    bool sd[4], any = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int d = (int)((a >> (8 * k)) & 0xFFu) - (int)((b >> (8 * k)) & 0xFFu);
+      sd[k] = k < n && c.gt((uint8_t)(d > 0 ? d : 0));
+      any = any || sd[k];
+    }
+    if (!any) return;
+    const int64_t gi = (int64_t)m.px_base + (int64_t)y * m.W + x;
+    int rf[4], r[4];
+    ccl::roots4_ro(c.LF, gi, n, rf);
+    ccl::roots4_ro(L2, gi, n, r);
+    bool kept = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k == 0 || rf[k] != rf[k - 1]) {
+        const int area = rf[k] < 0 || ccl::test_bit(c.outside, rf[k]) ? -1 : __ldg(c.A + rf[k]);
+        kept = area >= 0 && area >= c.lo && area < c.hi;
+      }
+      sd[k] = sd[k] && kept;
+      if (sd[k] && r[k] >= 0 && !(k > 0 && sd[k - 1] && r[k - 1] == r[k])) ccl::set_root_bit(bits, r[k]);
+    }
+  });
+}
 
 // ------------------------------------------------------------------------------------------
 // Output kernels (row grids over all images; a pixel's root is L[L[i]]).
@@ -512,6 +550,34 @@ __global__ void threshold_kernel(const T* in, int64_t pitch_in, uint8_t* out, in
       *(uchar4*)o = q;
     } else {
       for (int k = 0; k < 4 && x + k < W; ++k) o[k] = gt(r[k]) ? 255 : 0;
+    }
+  }
+}
+
+// 8- and 16-bit images whose rows allow it: 16 bytes of pixels per thread (four pixels per thread
+// took 205 us at 16384^2 u8, this 103).
+template <typename T>
+__global__ void threshold_wide_kernel(const T* in, int64_t pitch_in, uint8_t* out, int64_t pitch_out, int H, int W,
+                                      GtThr<T> gt) {
+  constexpr int V = 16 / sizeof(T);
+  const int x = V * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (x >= W) return;
+  for (int y = blockIdx.y; y < H; y += gridDim.y) {
+    const T* r = (const T*)((const char*)in + (int64_t)y * pitch_in) + x;
+    uint8_t* o = out + (int64_t)y * pitch_out + x;
+    if (x + V <= W) {
+      const uint4 v = *(const uint4*)r;
+      T e[V];
+      memcpy(e, &v, 16);
+      uint32_t q[V / 4];
+#pragma unroll
+      for (int k = 0; k < V / 4; ++k)
+        q[k] = (gt(e[4 * k]) ? 0xFFu : 0u) | (gt(e[4 * k + 1]) ? 0xFF00u : 0u) | (gt(e[4 * k + 2]) ? 0xFF0000u : 0u) |
+               (gt(e[4 * k + 3]) ? 0xFF000000u : 0u);
+      if constexpr (V == 16) *(uint4*)o = make_uint4(q[0], q[1], q[2], q[3]);
+      else *(uint2*)o = make_uint2(q[0], q[1]);
+    } else {
+      for (int k = 0; k < V && x + k < W; ++k) o[k] = gt(r[k]) ? 255 : 0;
     }
   }
 }
@@ -1220,6 +1286,11 @@ cudaError_t chain_impl(int dtype, const Plan& P, const Ws& w, int recon_conn, do
   return e;
 }
 
+// Quads of an image's rows start on 4-byte boundaries in both planes (u8).
+bool words_ok(const Img& m) {
+  return ((uintptr_t)m.plane % 4) == 0 && ((uintptr_t)m.aux % 4) == 0 && m.pitch % 4 == 0;
+}
+
 // The nucleus-candidate stage on one image (plane = rc_open, reconstructed in place; aux = rc):
 // (a) R = recon(rc_open, rc, 8); (b) bw1 = imfillHoles(D > g1, 4) and (c) bw1's 8-connected
 // components with their areas, from one labelling of D > g1 and its complement (the threshold
@@ -1246,8 +1317,8 @@ cudaError_t candidates_impl(const Plan& P, const Ws& w, double g1, double g2, in
   z.n[1] = 0;  // the status holds the reconstruction's
   if (e == cudaSuccess) e = ccl::label(ClsValleyAbove{gt2}, P.I, t, 8, sel, s, z);
   if (e == cudaSuccess)
-    e = launch_dependent(ccl::ccl_seed_quads<SeedCandidate>, qrb(t), dim3(256), s, P.I, t.rows, (const int*)w.R,
-                         SeedCandidate{gt2, w.L, w.A, lo, hi, outside}, w.bits);
+    e = launch_dependent(candidate_seeds_kernel, qrb(t), dim3(256), s, P.I, t.rows, (const int*)w.R,
+                         CandidateSeeds{gt2, w.L, w.A, lo, hi, outside, words_ok(P.I.one)}, w.bits);
   if (e == cudaSuccess)
     e = launch_dependent(candidates_out_kernel, qrb(t), dim3(256), s, P.I, t.rows, (const int*)w.R,
                          (const unsigned*)w.bits, rbc, out);
@@ -1654,6 +1725,14 @@ nsgb_status nsgb_threshold(int dtype, const void* in, uint8_t* out, int64_t rows
   dispatch_all(dtype, [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
     const GtThr<T> gt = GtThr<T>::make(thr);
+    if constexpr (sizeof(T) <= 2) {
+      constexpr int V = 16 / sizeof(T);
+      if ((uintptr_t)in % 16 == 0 && pitch_in % 16 == 0 && (uintptr_t)out % V == 0 && pitch_out % V == 0) {
+        const dim3 grid((unsigned)((cols + 256 * V - 1) / (256 * V)), ccl::row_blocks(H));
+        threshold_wide_kernel<T><<<grid, 256, 0, s>>>((const T*)in, pitch_in, out, pitch_out, H, W, gt);
+        return;
+      }
+    }
     if (vec) threshold_kernel<T, true><<<quad_grid(rows, cols), 256, 0, s>>>((const T*)in, pitch_in, out, pitch_out, H, W, gt);
     else threshold_kernel<T, false><<<quad_grid(rows, cols), 256, 0, s>>>((const T*)in, pitch_in, out, pitch_out, H, W, gt);
   });
