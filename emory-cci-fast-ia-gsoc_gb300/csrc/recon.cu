@@ -23,8 +23,9 @@
 //     alone if it is already queued (it has not loaded its halo yet and will read the new
 //     values).  A tile is therefore processed by one warp at a time and as soon as it can
 //     change; `pending` counts queued and running tiles and the kernel ends when it reaches 0.
-//     Stores and state reads / writes are separated by SC fences on both sides, so a neighbour
-//     either sees the new values or is re-run.
+//     A visit's stores are released by the atomics that mark its neighbours and acquired by the
+//     one that takes a tile (tilequeue.cuh), so a neighbour either sees the new values or is
+//     re-run.
 //
 // Every wait is bounded (status NSGB_ERR_TIMEOUT), and the per-visit sweep count and the
 // total number of visits are capped (status NSGB_ERR_NOT_CONVERGED).
@@ -113,8 +114,8 @@ __device__ __forceinline__ int clamped(int v, int n) { return min(max(v, 0), n -
 // Loads the word holding elements (y, x .. x+E-1), flipped into the working order; elements
 // outside the image read as LOW.  Outside, the nearest pixel is loaded and dropped: a load behind
 // a test of its coordinates waits for the one before it, and the halo of a tile is 16 loads (a
-// tile's loads took 17900 cycles of a 32-bit visit, most of them one halo load after another).  `coherent` selects L2-coherent loads for planes that other
-// warps write during the kernel.
+// tile's loads took 17900 cycles of a 32-bit visit, most of them one halo load after another).
+// `coherent` selects L2-coherent loads for planes that other warps write during the kernel.
 template <typename T>
 __device__ __forceinline__ uint32_t load_word(const T* base, int64_t pitch, int y, int x, int H, int W,
                                               bool fast, bool coherent, bool flip) {
