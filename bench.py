@@ -45,7 +45,7 @@ METRIC = "imreconstruct+bwlabel MPix/s, uint8 4096², plain vs batched GPU; % of
 # scan, assign), label/area/fill output.  See csrc/ops.cu chain_impl.  A tuned schedule with
 # streaming passes replaces recon init by its passes and two seed kernels (tuned_passes below).
 KERNELS_PER_CHAIN = 13
-KERNELS_PER_BATCH_CHAIN = 14
+KERNELS_PER_BATCH_CHAIN = 15
 E2E_LANES = 4  # streams the end-to-end steps rotate over
 
 
@@ -921,9 +921,9 @@ def bbox_section(args, dev, steps=20):
 
 # -- S1 after the colour steps: opening and nucleus-candidate stage ------------------------------
 # recon init + recon, bw1 filled and labelled at once (zeroing, local, merge, border walk,
-# parent join, flatten) + kept count, bw2 label (local, merge, flatten), seeds, output:
+# parent join, flatten) + kept count, bw2 label (zeroing, local, merge, flatten), seeds, output:
 # csrc/ops.cu candidates_impl
-CANDIDATE_KERNELS = 14
+CANDIDATE_KERNELS = 15
 OPEN_KERNELS = 2  # erosion, dilation (csrc/morph.cu)
 
 
@@ -1066,7 +1066,7 @@ def distance_section(args, dev, steps=20):
     px = H * W
     res = {"workload": f"{H}x{W} u8 mask (dark objects of the headline tile, mask < 128), basins output",
            "object_px": int(m_h.astype(bool).sum()), "ms": t, "ms_median": t_med, "mpix_s": px / 1e3 / t,
-           "gpu_launches_per_call": 3, "l2": "flushed before every step (512 MB write)"}
+           "gpu_launches_per_call": 5, "l2": "flushed before every step (512 MB write)"}
     if not args.no_cpu_baseline:
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
         import oracle
