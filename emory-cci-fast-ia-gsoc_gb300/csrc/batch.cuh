@@ -101,7 +101,7 @@ struct RColBase {
 // Totals of a batch, known on the host (grid sizes).
 struct BatchTotals {
   int n;
-  int64_t px;      // total pixels (< 2^31)
+  int64_t px;      // total pixels and the padding between images (< 2^31)
   int64_t b_words; // words of one bit plane over all images (rows x ceil(cols / 32))
   int f_tiles;     // flood tiles
   int r_tiles;     // reconstruction tiles
@@ -113,6 +113,7 @@ struct BatchTotals {
   int rows;        // total rows
   int max_w;       // widest image
   int perimeter_max;  // largest 2*(H+W)
+  bool tight;      // images follow each other in the label planes without alignment
 };
 
 }  // namespace nsgb

@@ -448,7 +448,8 @@ __global__ void label_out_kernel(Imgs I, int total_rows, const int* __restrict__
 }
 
 // The same for a batch, whose outputs are dense: an image is a line of pixels, and every quad of
-// it is aligned in the label plane (px_base is a multiple of 4) and in outputs that start aligned,
+// it is aligned in the label plane (px_base is a multiple of 4, or the quads are read one by one:
+// see batch_totals) and in outputs that start aligned,
 // whatever the width -- row by row an odd width left three rows of four to scalar accesses (71
 // Mpixel of uneven u8 tiles: 211 us row by row, 99 us along the line).  A CTA takes kLineBlocks
 // consecutive rank blocks of 1024 pixels and looks its image up once.
@@ -691,7 +692,7 @@ void add_image(Img& m, BatchTotals& t) {
   m.r_even_base = t.r_even;
   for (int c = 0; c < 3; ++c) m.r_col_base[c] = t.r_col[c];
   m.c_tile_base = t.c_tiles;
-  t.px = (t.px + 3) & ~(int64_t)3;  // four pixels of an image's label plane are one aligned load
+  if (!t.tight) t.px = (t.px + 3) & ~(int64_t)3;  // four pixels of an image's label plane are one aligned load
   m.px_base = (int)t.px;
   m.blk_base = t.blocks;
   m.row_base = t.rows;
@@ -1789,8 +1790,12 @@ nsgb_status nsgb_chain(int dtype, void* marker, const void* mask, int64_t rows, 
 
 namespace {
 
-bool batch_totals(int dtype, const nsgb_tile* tiles, int n, std::vector<Img>* imgs, BatchTotals* t) {
+// `tight`: without alignment of the images in the label planes.  A batch takes it when only the
+// padding would put it over the limit of 2^31 - 1 pixels (kernels check the alignment they use).
+bool batch_totals(int dtype, const nsgb_tile* tiles, int n, std::vector<Img>* imgs, BatchTotals* t,
+                  bool tight = false) {
   *t = BatchTotals{};
+  t->tight = tight;
   if (imgs) imgs->clear();
   const int esz = elem_size(dtype);
   if (!esz || !tiles || n <= 0) return false;
@@ -1803,7 +1808,7 @@ bool batch_totals(int dtype, const nsgb_tile* tiles, int n, std::vector<Img>* im
     m.fill = tl.fill_out;
     m.labels = tl.labels_out;
     m.area = tl.area_out;
-    if (t->px >= (int64_t)INT_MAX) return false;
+    if (t->px >= (int64_t)INT_MAX) return !tight && batch_totals(dtype, tiles, n, imgs, t, true);
     if (imgs) imgs->push_back(m);
   }
   return true;
