@@ -268,7 +268,7 @@ __device__ __forceinline__ int start_at(unsigned starts, int x) { return 31 - __
 // Bound: instructions issued (63% of cycles).  The kernel it replaced (a 256-thread CTA per tile,
 // unions, finds and area counts per pixel) issued about 5200 warp instructions per mixed tile,
 // this one 1200 (one class) to 1450 (two).  4096^2 u8, cold: two classes with areas 102 -> 38 us,
-// a 0 / 255 mask 76 -> 32 us; from a bit plane, 71 Mpixel of uneven tiles: 109 -> 49 us.
+// a 0 / 255 mask 76 -> 32 us; from a bit plane, 47 Mpixel of uneven tiles: 109 -> 70 us.
 template <class Cls, int CONN>
 __global__ void __launch_bounds__(32 * kLocalWarps) ccl_local(Cls cls, Imgs I, Forest f, int ntiles) {
   pdl_wait();
@@ -600,9 +600,9 @@ __device__ __forceinline__ void for_batch_quads(const Imgs& I, int total_rows, F
   });
 }
 
-// Roots of four consecutive pixels (L read-only): one 16-byte load when aligned.
-__device__ __forceinline__ void roots4_ro(const int* L, int64_t i, int n, int (&r)[4]) {
-  int l[4];
+// Label plane entries of four consecutive pixels (L read-only; -1 from n on): one 16-byte load
+// when aligned.
+__device__ __forceinline__ void labels4_ro(const int* L, int64_t i, int n, int (&l)[4]) {
   if (n == 4 && ((i & 3) == 0)) {
     const int4 v = __ldg((const int4*)(L + i));
     l[0] = v.x, l[1] = v.y, l[2] = v.z, l[3] = v.w;
@@ -610,6 +610,12 @@ __device__ __forceinline__ void roots4_ro(const int* L, int64_t i, int n, int (&
 #pragma unroll
     for (int k = 0; k < 4; ++k) l[k] = k < n ? __ldg(L + i + k) : -1;
   }
+}
+
+// Roots of four consecutive pixels (L read-only).
+__device__ __forceinline__ void roots4_ro(const int* L, int64_t i, int n, int (&r)[4]) {
+  int l[4];
+  labels4_ro(L, i, n, l);
 #pragma unroll
   for (int k = 0; k < 4; ++k) r[k] = l[k] < 0 ? -1 : (k > 0 && l[k] == l[k - 1] ? -2 : __ldg(L + l[k]));
 #pragma unroll

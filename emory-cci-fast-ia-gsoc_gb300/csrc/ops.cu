@@ -450,8 +450,8 @@ __global__ void label_out_kernel(Imgs I, int total_rows, const int* __restrict__
 // The same for a batch, whose outputs are dense: an image is a line of pixels, and every quad of
 // it is aligned in the label plane (px_base is a multiple of 4, or the quads are read one by one:
 // see batch_totals) and in outputs that start aligned,
-// whatever the width -- row by row an odd width left three rows of four to scalar accesses (71
-// Mpixel of uneven u8 tiles: 211 us row by row, 99 us along the line).  A CTA takes kLineBlocks
+// whatever the width -- row by row an odd width left three rows of four to scalar accesses (47
+// Mpixel of uneven u8 tiles: 211 us row by row, 98 us along the line).  A CTA takes kLineBlocks
 // consecutive rank blocks of 1024 pixels and looks its image up once.
 constexpr int kLineBlocks = 4;
 template <bool RELABEL, bool AREA, bool FILLED>
@@ -1084,15 +1084,26 @@ __global__ void __launch_bounds__(1024) seed_check_kernel(Imgs I, const int* __r
 // The start: the image on the border, max elsewhere, and the level on the pixels joined to the
 // border at it.  With `c` the level just tried is added (the first one used writes the whole plane);
 // without, the plain marker is written unless a level was used (`last`).  Four pixels per thread.
+// Bound: the latency of three dependent loads a quad (label, root, bit).  The loads of each step are
+// unconditional (clamped) so that they go out together, and a CTA takes consecutive rows of the one
+// image, so that the rows of a labelling tile find its roots in L1: 16384^2 u8, a noisy level,
+// 635 -> 558 us by the first and 378 us by both.
 template <typename T>
-__global__ void __launch_bounds__(256) seed_marker_kernel(Imgs I, int total_rows, const int* __restrict__ L,
+__global__ void __launch_bounds__(256) seed_marker_kernel(Imgs I, const int* __restrict__ L,
                                                           const unsigned* __restrict__ bits, T* out,
                                                           const SeedCtl* __restrict__ c, bool last) {
   const int used = c ? c->used + (last ? c->use : 0) : 0;
   if (c && (last ? used != 0 : c->use == 0)) return;
   const bool joined = c && !last, add = joined && used != 0;
   const int level = joined ? c->level : 0;
-  ccl::for_batch_quads(I, total_rows, [&](const Img& m, int y, int x, int n) {
+  const Img& m = I.one;
+  const int x = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (x >= m.W) return;
+  const int n = min(4, m.W - x);
+  const int per = (m.H + (int)gridDim.y - 1) / (int)gridDim.y;
+  const int y0 = (int)blockIdx.y * per, y1 = min(m.H, y0 + per);
+#pragma unroll 2
+  for (int y = y0; y < y1; ++y) {
     const T* in = pxp<T>(m.plane, m.pitch, y, x);
     T* o = pxp<T>(out, m.pitch, y, x);
     const bool vec = n == 4 && ((uintptr_t)o & (4 * sizeof(T) - 1)) == 0;
@@ -1106,17 +1117,19 @@ __global__ void __launch_bounds__(256) seed_marker_kernel(Imgs I, int total_rows
       } else {
         for (int k = 0; k < n; ++k) v[k] = o[k];
       }
-      if (v[0] != kMax && v[1] != kMax && v[2] != kMax && v[3] != kMax) return;
+      if (v[0] != kMax && v[1] != kMax && v[2] != kMax && v[3] != kMax) continue;
     }
     if (joined) {
-      int r[4];
-      bool on[4];
-      ccl::roots4_ro(L, (int64_t)y * m.W + x, n, r);
+      int l[4], r[4];
+      unsigned word[4];
+      ccl::labels4_ro(L, (int64_t)y * m.W + x, n, l);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        on[k] = k > 0 && r[k] == r[k - 1] ? on[k - 1] : r[k] >= 0 && ccl::test_bit(bits, r[k]);
-        if (on[k] && v[k] == kMax) v[k] = (T)level;
-      }
+      for (int k = 0; k < 4; ++k) r[k] = __ldg(L + max(l[k], 0));
+#pragma unroll
+      for (int k = 0; k < 4; ++k) word[k] = __ldg(bits + (max(r[k], 0) >> 5));
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (l[k] >= 0 && ((word[k] >> (r[k] & 31)) & 1u) && v[k] == kMax) v[k] = (T)level;
     }
     if (!add) {
       if (y == 0 || y == m.H - 1) {
@@ -1131,7 +1144,7 @@ __global__ void __launch_bounds__(256) seed_marker_kernel(Imgs I, int total_rows
     } else {
       for (int k = 0; k < n; ++k) o[k] = v[k];
     }
-  });
+  }
 }
 
 // The fill's start in `out` (see above).  P: the image as the plan's plane.  The crops live in
@@ -1175,11 +1188,11 @@ cudaError_t fill_start(int dtype, const Plan& P, const Ws& w, T* out, int conn, 
         if (e != cudaSuccess) return e;
         seed_border_kernel<T><<<64, 256, 0, s>>>(P.I, w.L, cls, w.bits);
         seed_check_kernel<T><<<1, 1024, 0, s>>>(P.I, w.L, cls, w.bits, c);
-        seed_marker_kernel<T><<<rows, 256, 0, s>>>(P.I, P.t.rows, w.L, w.bits, out, c, false);
+        seed_marker_kernel<T><<<rows, 256, 0, s>>>(P.I, w.L, w.bits, out, c, false);
       }
     }
   }
-  seed_marker_kernel<T><<<rows, 256, 0, s>>>(P.I, P.t.rows, w.L, w.bits, out, c, true);
+  seed_marker_kernel<T><<<rows, 256, 0, s>>>(P.I, w.L, w.bits, out, c, true);
   return cudaGetLastError();
 }
 
