@@ -473,6 +473,11 @@ class BatchPlan:
         self._ws = torch.empty(need + 256, dtype=torch.uint8, device=self.masks[0].device)
         ptr = (self._ws.data_ptr() + 255) & ~255
         self.batch = _ffi.Batch()
+        # The table is written on the default stream; on another one, work queued earlier may still be
+        # using the memory that the workspace was given.
+        stream = torch.cuda.current_stream()
+        if stream.cuda_stream != 0:
+            stream.synchronize()
         _ffi.check(lib.nsgb_batch_prepare(dt, tiles, len(markers), ptr, need, C.byref(self.batch)), "batch_prepare")
         self.n = len(markers)
 

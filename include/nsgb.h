@@ -283,7 +283,8 @@ typedef struct {
 size_t nsgb_batch_workspace_size(int dtype, const nsgb_tile* tiles, int n_tiles);
 /* Writes the batch's image table into `ws` (synchronous) and fills `batch`.  Afterwards the
  * batch calls below enqueue kernels only, so they can be replayed many times (and recorded
- * once) with the same tiles. */
+ * once) with the same tiles.  It works on the default stream and does not wait for a non-blocking
+ * stream: no work of such a stream may still use `ws`. */
 nsgb_status nsgb_batch_prepare(int dtype, const nsgb_tile* tiles, int n_tiles, void* ws, size_t ws_bytes,
                                nsgb_batch* batch);
 /* nsgb_chain on every tile of the batch; n_labels / n_kept: optional host arrays of n_tiles
