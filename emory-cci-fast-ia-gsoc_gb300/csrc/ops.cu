@@ -5,6 +5,7 @@
 // point.
 #include <cuda_runtime.h>
 #include <limits.h>
+#include <stddef.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -2320,8 +2321,13 @@ __device__ __forceinline__ Fix128 far_sum(const GradArgs& a, int c, int64_t gq) 
 // to float with one rounding (the scale is a power of two).  Tiles outside that range are listed
 // for grad_wide_tiles.
 constexpr int kSpan = 29;
+struct alignas(16) GradLimbs {  // cleared 16 bytes at a time
+  int v[2][3][kGradPx];
+};
+static_assert(alignof(GradLimbs) >= alignof(uint4) && sizeof(GradLimbs) % sizeof(uint4) == 0, "cleared as uint4");
 __global__ void __launch_bounds__(kGradThreads) grad_tiles_kernel(GradArgs a) {
-  __shared__ int limb[2][3][kGradPx];
+  __shared__ GradLimbs limbs;
+  int (&limb)[2][3][kGradPx] = limbs.v;
   __shared__ uint16_t list[2 * kGradPx];  // class * kGradPx + pixel: sums with a far part
   __shared__ int listed, s_lo[kGradThreads / 32], s_hi[kGradThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2338,7 +2344,7 @@ __global__ void __launch_bounds__(kGradThreads) grad_tiles_kernel(GradArgs a) {
     g[k] = k < rows_in ? __ldg((const uint32_t*)((const char*)a.g + at + k * a.pitch)) : 0u;
   }
   for (int i = threadIdx.x; i < 2 * 3 * kGradPx / 4; i += kGradThreads)
-    ((uint4*)limb)[i] = make_uint4(0u, 0u, 0u, 0u);
+    ((uint4*)&limbs)[i] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
   for (int k = 0; k < kGradRows; ++k) {
     const int ex = (g[k] >> 23) & 0xFF;
@@ -2426,12 +2432,13 @@ __global__ void __launch_bounds__(kGradThreads) grad_tiles_kernel(GradArgs a) {
 // are their slot.
 constexpr int kLimbs = 6, kLimbBits = 21;
 constexpr uint32_t kNoGrad = 0xFFFFFFFFu;  // a NaN: never a gradient in a slot
-struct GradTile {
+struct alignas(16) GradTile {  // slots and limbs are set 16 bytes at a time
   uint32_t slot[2][kGradPx];
   int limb[2][kLimbs][kGradPx];
   uint16_t list[2 * kGradPx];  // class * kGradPx + pixel
   int listed;
 };
+static_assert(alignof(GradTile) >= alignof(uint4) && offsetof(GradTile, limb) % sizeof(uint4) == 0, "set as uint4");
 
 __device__ __forceinline__ void limb_add(int (*limb)[kGradPx], int i, float g) {
   const uint32_t b = __float_as_uint(g), ex = (b >> 23) & 0xFFu;
