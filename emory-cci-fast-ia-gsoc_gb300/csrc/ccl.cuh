@@ -133,14 +133,11 @@ __device__ __forceinline__ void g_union(int* L, int a, int b) {
 // root is px_base + the smallest raster index of the component.  A (optional) holds the pixel
 // count of each local root, then of each global root.  `roots` lists the local roots,
 // `nroots` counts them.
-// `skip` (optional): a device word; while it is not zero the labelling kernels return at once.
 struct Forest {
   int* L;
   int* A;
   int* roots;
   int* nroots;
-  const int* skip = nullptr;
-  __device__ bool skipped() const { return skip && __ldcg(skip) != 0; }
 };
 
 __device__ __forceinline__ int root_of(const int* L, int64_t i) {
@@ -155,19 +152,22 @@ __device__ __forceinline__ int root_of_ro(const int* L, int64_t i) {
   return l < 0 ? -1 : __ldg(L + l);
 }
 
-// Labelling tile of CTA `b`: image, tile origin.
+// Labelling tile `b`: image, tile origin.
 struct TileAt {
   Img m;
   int x0, y0;
 };
-__device__ __forceinline__ TileAt tile_at(const Imgs& I, int b) {
+__device__ __forceinline__ TileAt tile_in(const Img& m, int b) {
   TileAt t;
-  t.m = img_at(I, img_of_tile(I, b, I.c_img, I.c_per, CTileBase()));
+  t.m = m;
   const int lt = b - t.m.c_tile_base;
   const int ty = lt / t.m.c_tiles_x;
   t.x0 = (lt - ty * t.m.c_tiles_x) * kTile;
   t.y0 = ty * kTile;
   return t;
+}
+__device__ __forceinline__ TileAt tile_at(const Imgs& I, int b) {
+  return tile_in(img_at(I, img_of_tile(I, b, I.c_img, I.c_per, CTileBase())), b);
 }
 
 // Width of the class values a classifier produces: 8 bits unless it declares `class_t`
@@ -269,18 +269,11 @@ __device__ __forceinline__ int start_at(unsigned starts, int x) { return 31 - __
 // unions, finds and area counts per pixel) issued about 5200 warp instructions per mixed tile,
 // this one 1200 (one class) to 1450 (two).  4096^2 u8, cold: two classes with areas 102 -> 38 us,
 // a 0 / 255 mask 76 -> 32 us; from a bit plane, 47 Mpixel of uneven tiles: 109 -> 70 us.
+//
+// `s` (1024 words) and `starts` (32) are the warp's own shared memory.
 template <class Cls, int CONN>
-__global__ void __launch_bounds__(32 * kLocalWarps) ccl_local(Cls cls, Imgs I, Forest f, int ntiles) {
-  pdl_wait();
-  pdl_release();
-  __shared__ int s_nodes[kLocalWarps][kTile * kTile];
-  __shared__ unsigned s_starts[kLocalWarps][kTile];
-  const int b = blockIdx.x * kLocalWarps + (threadIdx.x >> 5);
-  if (b >= ntiles || f.skipped()) return;  // whole warp; the warps of a CTA are independent
-  int* s = s_nodes[threadIdx.x >> 5];
-  unsigned* starts = s_starts[threadIdx.x >> 5];
+__device__ __forceinline__ void local_tile(const Cls& cls, const TileAt& T, const Forest& f, int* s, unsigned* starts) {
   const int lane = threadIdx.x & 31;
-  const TileAt T = tile_at(I, b);
   const int x0 = T.x0, y0 = T.y0, W = T.m.W, pb = T.m.px_base;
   const int gx = x0 + lane;
   const unsigned cols_in = W - x0 >= 32 ? 0xFFFFFFFFu : (1u << (W - x0)) - 1u;
@@ -447,6 +440,17 @@ __global__ void __launch_bounds__(32 * kLocalWarps) ccl_local(Cls cls, Imgs I, F
   }
 }
 
+template <class Cls, int CONN>
+__global__ void __launch_bounds__(32 * kLocalWarps) ccl_local(Cls cls, Imgs I, Forest f, int ntiles) {
+  pdl_wait();
+  pdl_release();
+  __shared__ int s_nodes[kLocalWarps][kTile * kTile];
+  __shared__ unsigned s_starts[kLocalWarps][kTile];
+  const int b = blockIdx.x * kLocalWarps + (threadIdx.x >> 5);
+  if (b >= ntiles) return;  // whole warp; the warps of a CTA are independent
+  local_tile<Cls, CONN>(cls, tile_at(I, b), f, s_nodes[threadIdx.x >> 5], s_starts[threadIdx.x >> 5]);
+}
+
 // Joins runs across tile edges.  Two warps per labelling tile: warp 0 takes the bottom edge
 // (row y0+31 against row y0+32), warp 1 the right edge (column x0+31 against column x0+32, the
 // same logic transposed).  With `a` = the pixel on this side and `b` its partner across the
@@ -454,17 +458,9 @@ __global__ void __launch_bounds__(32 * kLocalWarps) ccl_local(Cls cls, Imgs I, F
 // where a run on the far side starts or where a near-side run starts under a far-side run,
 // plus the two diagonal ends of each far-side run for 8-connectivity.
 template <class Cls, int CONN>
-__global__ void __launch_bounds__(64 * kMergeTiles) ccl_merge(Cls cls, Imgs I, Forest f, int ntiles) {
-  pdl_wait();
-  pdl_release();
-  if (f.skipped()) return;
-  int* __restrict__ const L = f.L;
-  const int b = blockIdx.x * kMergeTiles + (threadIdx.x >> 6);
-  if (b >= ntiles) return;
-  const TileAt T = tile_at(I, b);
+__device__ __forceinline__ void merge_edge(const Cls& cls, const TileAt& T, int* L, bool bottom) {
   const int x0 = T.x0, y0 = T.y0, H = T.m.H, W = T.m.W, pb = T.m.px_base;
   const int lane = threadIdx.x & 31;
-  const bool bottom = ((threadIdx.x >> 5) & 1) == 0;
   // coordinates of the near pixel (a) and the far pixel (b) for this lane
   int ay, ax, by, bx;
   if (bottom) {
@@ -510,14 +506,20 @@ __global__ void __launch_bounds__(64 * kMergeTiles) ccl_merge(Cls cls, Imgs I, F
   }
 }
 
+template <class Cls, int CONN>
+__global__ void __launch_bounds__(64 * kMergeTiles) ccl_merge(Cls cls, Imgs I, Forest f, int ntiles) {
+  pdl_wait();
+  pdl_release();
+  const int b = blockIdx.x * kMergeTiles + (threadIdx.x >> 6);
+  if (b < ntiles) merge_edge<Cls, CONN>(cls, tile_at(I, b), f.L, ((threadIdx.x >> 5) & 1) == 0);
+}
+
 // Every local root points directly at its global root; local-root areas move into the root.
 // Four list entries per thread and iteration, their loads issued together: most local roots
 // are global roots already (one load to see it), so the kernel is load-latency bound.  The
 // area adds of a warp are summed per root first (one atomic per root and warp): the local
 // roots of a giant component, one per labelling tile, all add into the same word.
-static __global__ void ccl_flatten_roots(Forest f, int max_roots) {
-  pdl_wait();
-  pdl_release();
+__device__ __forceinline__ void flatten_roots(const Forest& f, int max_roots) {
   const int n = min(__ldcg(f.nroots), max_roots);
   const int stride = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
@@ -546,6 +548,12 @@ static __global__ void ccl_flatten_roots(Forest f, int max_roots) {
       }
     }
   }
+}
+
+static __global__ void ccl_flatten_roots(Forest f, int max_roots) {
+  pdl_wait();
+  pdl_release();
+  flatten_roots(f, max_roots);
 }
 
 __device__ __forceinline__ void set_root_bit(unsigned* bits, int r) {

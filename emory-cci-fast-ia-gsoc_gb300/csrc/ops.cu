@@ -22,6 +22,7 @@
 #include "ccl.cuh"
 #include "common.cuh"
 #include "edt.cuh"
+#include "fillstart.cuh"
 #include "morph.cuh"
 #include "recon.cuh"
 
@@ -762,7 +763,7 @@ struct Ws {
   int* r_img;  // batches: image of every reconstruction tile
   int* c_img;  // batches: image of every labelling tile
   size_t bits_bytes;
-  ccl::Forest forest(bool areas) const { return ccl::Forest{L, areas ? A : nullptr, roots, nroots, nullptr}; }
+  ccl::Forest forest(bool areas) const { return ccl::Forest{L, areas ? A : nullptr, roots, nroots}; }
 };
 
 Ws carve(void* ws, const BatchTotals& t) {
@@ -895,308 +896,6 @@ BatchTotals stacked_totals(const BatchTotals& one, int64_t n) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Grayscale hole filling: a start near the end.
-//
-// The fill is the erosion reconstruction of (image on the border, max inside).  Started from that
-// marker, a front crosses the whole image tile by tile, and the time is that chain of dependent
-// tile visits (16384^2 u8: 14.4 ms, 3% of the copy bandwidth).  But any start between the marker
-// and the result gives the same result, and on an image with few grey levels most of the result
-// is known early: away from the border a pixel fills to the larger of its own value and the level at
-// which the image conducts from side to side (its percolation level), since only near the border
-// is there a lower way out.  So:
-//   (1) the level is estimated on 12 x 12 crops of 64 x 64 pixels: the lowest level at which a
-//       crop is crossed from left to right is the smallest result of a fill from its left column (one
-//       batched reconstruction);
-//   (2) up to three levels in rising order, from the lower quartile of the crops' on, are tried:
-//       the pixels at or below the level are labelled (union-find: no chain) and the components that
-//       touch the border are marked.  A level conducts, and
-//       no further one is tried, when they hold half of the pixels at or below it on a grid over the
-//       image's inner half;
-//   (3) the start is the lowest level tried at which a pixel is marked (it is joined to a border
-//       pixel through pixels at or below the level, so its result is at most the level), and the
-//       marker elsewhere.
-// The reconstruction then only works near the border and in closed pockets.  A level above the
-// right one would leave the whole chain to do, and with many grey levels (a conducting level
-// shared by no two crops) there is no exact level to find: more than kSeedDistinct distinct crop
-// levels, or no level that conducts, and the start is the marker as before.
-constexpr int kCropGrid = 12, kCrops = kCropGrid * kCropGrid, kCrop = 64;
-constexpr int kSeedLevels = 3, kSeedDistinct = 36;
-constexpr int kSeedGrid = 64;  // check points per side
-// Smaller sides keep the plain marker: 1024^2 u8 takes 0.61 ms from it and 0.59 from an estimated
-// start, 1300^2 u16 0.93 and 0.61, 768^2 u8 0.41 and 0.50.
-constexpr int64_t kSeedMinSide = 1280;
-constexpr int kSeedSamples = 1024, kSeedMany = 512;
-
-struct SeedCtl {  // device
-  int skip;       // the kernels of the current level return at once
-  int found;      // a level conducts all through: no further ones are tried
-  int level;      // level being tried
-  int use;        // it was labelled: its marked pixels go into the start
-  int used;       // levels that the start holds so far
-  int n;          // levels to try
-  int many;       // the image has many grey levels: none is tried
-  int levels[kSeedLevels];
-};
-
-template <typename T>
-struct ClsAtMost {
-  static constexpr ccl::ClassKind kKind = ccl::kOneClass;
-  const SeedCtl* c;
-  __device__ uint32_t operator()(const Img& m, int y, int x) const {
-    return (int)px<T>(m.plane, m.pitch, y, x) <= c->level ? 1u : 0u;
-  }
-};
-
-// Many grey levels?  (16-bit and 32-bit images: more than half of 1024 pixels on a grid differ
-// from all others; the crops are then blank, which costs one visit each instead of the chain.)
-template <typename T>
-__global__ void __launch_bounds__(kSeedSamples) seed_sample_kernel(const T* image, int64_t pitch, int H, int W, SeedCtl* c) {
-  __shared__ int v[kSeedSamples];
-  __shared__ int s_distinct;
-  const int k = threadIdx.x, n = 32;
-  if (k == 0) s_distinct = 0;
-  v[k] = (int)px<T>(image, pitch, (int)(((int64_t)H * (2 * (k / n) + 1)) / (2 * n)),
-                    (int)(((int64_t)W * (2 * (k % n) + 1)) / (2 * n)));
-  __syncthreads();
-  if (sizeof(T) > 1) {
-    const int own = v[k];
-    bool first = true;
-    for (int j = 0; j < k; ++j) first = first && v[j] != own;
-    const int count = __popc(__ballot_sync(NSGB_FULL, first));
-    if ((k & 31) == 0) atomicAdd(&s_distinct, count);
-  }
-  __syncthreads();
-  if (k == 0) c->many = s_distinct > kSeedMany;
-}
-
-// Crop k into its plane (mask) and its marker: the image in the left column, max elsewhere.
-template <typename T>
-__global__ void seed_crops_kernel(const T* image, int64_t pitch, int H, int W, T* marker, T* mask,
-                                  const SeedCtl* c) {
-  const int k = blockIdx.y, cy = k / kCropGrid, cx = k - cy * kCropGrid;
-  const int y0 = (int)(((int64_t)(H - kCrop) * (2 * cy + 1)) / (2 * kCropGrid));
-  const int x0 = (int)(((int64_t)(W - kCrop) * (2 * cx + 1)) / (2 * kCropGrid));
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kCrop * kCrop; i += gridDim.x * blockDim.x) {
-    const int y = i / kCrop, x = i - y * kCrop;
-    const T v = c->many ? (T)0 : px<T>(image, pitch, y0 + y, x0 + x);
-    mask[(int64_t)k * kCrop * kCrop + i] = v;
-    marker[(int64_t)k * kCrop * kCrop + i] = x == 0 || c->many ? v : std::numeric_limits<T>::max();
-  }
-}
-
-// The crops' levels, in order, and the levels to try.  One CTA of kCrops threads or more.
-template <typename T>
-__global__ void seed_levels_kernel(const T* filled, SeedCtl* c) {
-  __shared__ int level[kCrops], sorted[kCrops];
-  const int k = threadIdx.x;
-  if (k < kCrops) {
-    int v = INT_MAX;
-    for (int y = 0; y < kCrop; ++y)
-      v = min(v, (int)__ldcg(filled + (int64_t)k * kCrop * kCrop + y * kCrop + kCrop - 1));
-    level[k] = v;
-  }
-  __syncthreads();
-  if (k < kCrops) {
-    int r = 0;
-    for (int j = 0; j < kCrops; ++j) r += level[j] < level[k] || (level[j] == level[k] && j < k);
-    sorted[r] = level[k];
-  }
-  __syncthreads();
-  if (k == 0) {
-    int distinct = 1;
-    for (int j = 1; j < kCrops; ++j) distinct += sorted[j] != sorted[j - 1];
-    int n = 0;
-    if (distinct <= kSeedDistinct && !c->many) {
-      c->levels[n++] = sorted[kCrops / 4];
-      for (int j = kCrops / 4 + 1; j < kCrops && n < kSeedLevels; ++j)
-        if (sorted[j] != c->levels[n - 1]) c->levels[n++] = sorted[j];
-    }
-    c->n = n;
-    c->found = 0;
-    c->use = 0;
-    c->used = 0;
-  }
-}
-
-// Level k becomes the current one (skipped once a level conducts, or if there is none); the
-// root list and the bitmap are cleared.
-__global__ void seed_begin_kernel(SeedCtl* c, int k, int* nroots, unsigned* bits, int words) {
-  const bool skip = c->found != 0 || k >= c->n;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (!skip)
-    for (int j = i; j < words; j += gridDim.x * blockDim.x) bits[j] = 0u;
-  if (i == 0) {
-    c->skip = skip ? 1 : 0;
-    c->used += c->use;
-    c->use = 0;
-    if (!skip) {
-      c->level = c->levels[k];
-      *nroots = 0;
-    }
-  }
-}
-
-template <typename T>
-__global__ void seed_border_kernel(Imgs I, const int* __restrict__ L, ClsAtMost<T> cls, unsigned* bits) {
-  if (cls.c->skip) return;
-  const Img& m = I.one;
-  const int per = 2 * m.W + 2 * m.H;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < per; k += gridDim.x * blockDim.x) {
-    int y, x;
-    ccl::border_pixel(k, m.H, m.W, y, x);
-    if (!cls(m, y, x)) continue;
-    const int r = ccl::root_of(L, (int64_t)y * m.W + x);
-    if (r >= 0) ccl::set_root_bit(bits, r);
-  }
-}
-
-// Does the current level conduct?  One CTA.
-template <typename T>
-__global__ void __launch_bounds__(1024) seed_check_kernel(Imgs I, const int* __restrict__ L, ClsAtMost<T> cls,
-                                                          const unsigned* bits, SeedCtl* c) {
-  __shared__ int s_low, s_joined;
-  if (c->skip) return;
-  if (threadIdx.x == 0) s_low = s_joined = 0;
-  __syncthreads();
-  const Img& m = I.one;
-  int low = 0, joined = 0;
-  for (int k = threadIdx.x; k < kSeedGrid * kSeedGrid; k += blockDim.x) {
-    const int gy = k / kSeedGrid, gx = k - gy * kSeedGrid;
-    const int y = m.H / 4 + (int)(((int64_t)(m.H / 2) * gy) / kSeedGrid);
-    const int x = m.W / 4 + (int)(((int64_t)(m.W / 2) * gx) / kSeedGrid);
-    if (!cls(m, y, x)) continue;
-    ++low;
-    const int r = ccl::root_of(L, (int64_t)y * m.W + x);
-    joined += r >= 0 && ((__ldcg(bits + (r >> 5)) >> (r & 31)) & 1u);
-  }
-  low = __reduce_add_sync(NSGB_FULL, low);
-  joined = __reduce_add_sync(NSGB_FULL, joined);
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&s_low, low);
-    atomicAdd(&s_joined, joined);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    c->use = 1;
-    if (s_low > 0) c->found = 2 * s_joined >= s_low;
-  }
-}
-
-// The start: the image on the border, max elsewhere, and the level on the pixels joined to the
-// border at it.  With `c` the level just tried is added (the first one used writes the whole plane);
-// without, the plain marker is written unless a level was used (`last`).  Four pixels per thread.
-// Bound: the latency of three dependent loads a quad (label, root, bit).  The loads of each step are
-// unconditional (clamped) so that they go out together, and a CTA takes consecutive rows of the one
-// image, so that the rows of a labelling tile find its roots in L1: 16384^2 u8, a noisy level,
-// 635 -> 558 us by the first and 378 us by both.
-template <typename T>
-__global__ void __launch_bounds__(256) seed_marker_kernel(Imgs I, const int* __restrict__ L,
-                                                          const unsigned* __restrict__ bits, T* out,
-                                                          const SeedCtl* __restrict__ c, bool last) {
-  const int used = c ? c->used + (last ? c->use : 0) : 0;
-  if (c && (last ? used != 0 : c->use == 0)) return;
-  const bool joined = c && !last, add = joined && used != 0;
-  const int level = joined ? c->level : 0;
-  const Img& m = I.one;
-  const int x = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-  if (x >= m.W) return;
-  const int n = min(4, m.W - x);
-  const int per = (m.H + (int)gridDim.y - 1) / (int)gridDim.y;
-  const int y0 = (int)blockIdx.y * per, y1 = min(m.H, y0 + per);
-#pragma unroll 2
-  for (int y = y0; y < y1; ++y) {
-    const T* in = pxp<T>(m.plane, m.pitch, y, x);
-    T* o = pxp<T>(out, m.pitch, y, x);
-    const bool vec = n == 4 && ((uintptr_t)o & (4 * sizeof(T) - 1)) == 0;
-    constexpr T kMax = std::numeric_limits<T>::max();
-    T v[4] = {kMax, kMax, kMax, kMax};
-    if (add) {
-      if (vec) {
-        const Vec4<T> q = *(const Vec4<T>*)o;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = q.v[k];
-      } else {
-        for (int k = 0; k < n; ++k) v[k] = o[k];
-      }
-      if (v[0] != kMax && v[1] != kMax && v[2] != kMax && v[3] != kMax) continue;
-    }
-    if (joined) {
-      int l[4], r[4];
-      unsigned word[4];
-      ccl::labels4_ro(L, (int64_t)y * m.W + x, n, l);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) r[k] = __ldg(L + max(l[k], 0));
-#pragma unroll
-      for (int k = 0; k < 4; ++k) word[k] = __ldg(bits + (max(r[k], 0) >> 5));
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (l[k] >= 0 && ((word[k] >> (r[k] & 31)) & 1u) && v[k] == kMax) v[k] = (T)level;
-    }
-    if (!add) {
-      if (y == 0 || y == m.H - 1) {
-        for (int k = 0; k < n; ++k) v[k] = in[k];
-      } else {
-        if (x == 0) v[0] = in[0];
-        if (x + n == m.W) v[n - 1] = in[n - 1];
-      }
-    }
-    if (vec) {
-      *(Vec4<T>*)o = Vec4<T>{v[0], v[1], v[2], v[3]};
-    } else {
-      for (int k = 0; k < n; ++k) o[k] = v[k];
-    }
-  }
-}
-
-// The fill's start in `out` (see above).  P: the image as the plan's plane.  The crops live in
-// the workspace planes A (markers) and R (masks), which the fill does not otherwise use, the image
-// table and the control words in `tmp`'s plane F.
-template <typename T>
-cudaError_t fill_start(int dtype, const Plan& P, const Ws& w, T* out, int conn, cudaStream_t s) {
-  const Img& m = P.I.one;
-  const bool seed = std::is_integral<T>::value && m.H >= kSeedMinSide && m.W >= kSeedMinSide;
-  SeedCtl* const c = seed ? (SeedCtl*)w.F : nullptr;
-  // few CTAs of many rows: most launches of the marker kernel find nothing to do
-  const dim3 rows(qrb(P.t).x, seed ? 1024 : qrb(P.t).y);
-  cudaError_t e = cudaSuccess;
-  if constexpr (std::is_integral<T>::value) {
-    if (seed) {
-      T *marker = (T*)w.A, *mask = (T*)w.R;
-      seed_sample_kernel<T><<<1, kSeedSamples, 0, s>>>((const T*)m.plane, m.pitch, m.H, m.W, c);
-      seed_crops_kernel<T><<<dim3(4, kCrops), 256, 0, s>>>((const T*)m.plane, m.pitch, m.H, m.W, marker, mask, c);
-      const Plan C1 = single_plan(dtype, marker, mask, kCrop, kCrop, kCrop * sizeof(T));
-      Plan C = C1;
-      C.t = stacked_totals(C1.t, kCrops);
-      C.I.n = kCrops;
-      C.I.d = (Img*)(w.F + 256);
-      C.I.r_per = C1.t.r_tiles;
-      C.I.c_per = C1.t.c_tiles;
-      stack_table_kernel<<<(kCrops + 127) / 128, 128, 0, s>>>(C1.I.one, kCrops, (int64_t)kCrop * kCrop * sizeof(T), C1.t,
-                                                              (Img*)(w.F + 256));
-      e = cudaGetLastError();
-      if (e == cudaSuccess)
-        e = recon_launch_batch(dtype, C.I, C.t.r_tiles, conn, true, false, w.recon, s, 0, 0, 0, 0, -1, 0, 0,
-                               (long long)C.t.px, 0);
-      if (e != cudaSuccess) return e;
-      seed_levels_kernel<T><<<1, 256, 0, s>>>(marker, c);
-      const ClsAtMost<T> cls{c};
-      ccl::Forest f = w.forest(false);
-      f.skip = &c->skip;
-      const int words = (int)(w.bits_bytes / sizeof(unsigned));
-      for (int k = 0; k < kSeedLevels; ++k) {
-        seed_begin_kernel<<<ccl::flat_grid(words), 256, 0, s>>>(c, k, w.nroots, w.bits, words);
-        e = ccl::label(cls, P.I, P.t, conn, f, s);
-        if (e != cudaSuccess) return e;
-        seed_border_kernel<T><<<64, 256, 0, s>>>(P.I, w.L, cls, w.bits);
-        seed_check_kernel<T><<<1, 1024, 0, s>>>(P.I, w.L, cls, w.bits, c);
-        seed_marker_kernel<T><<<rows, 256, 0, s>>>(P.I, w.L, w.bits, out, c, false);
-      }
-    }
-  }
-  seed_marker_kernel<T><<<rows, 256, 0, s>>>(P.I, w.L, w.bits, out, c, true);
-  return cudaGetLastError();
-}
-
 // The single-tile / batched chain on a prepared plan: (a) reconstruction in place,
 // (b)+(c) threshold fused into the binary hole fill, (d)+(e) one labelling of the filled image
 // for both the raster relabel and the areas.  Counts land in w.counts (2 per image).
@@ -1327,7 +1026,7 @@ cudaError_t candidates_impl(const Plan& P, const Ws& w, double g1, double g2, in
                           w.bits_bytes, s, true, ccl::ZeroSpans{{nullptr, nullptr, (unsigned*)w.counts, nullptr}, {0, 0, 2 * t.n, 0}});
   if (e == cudaSuccess)
     e = ccl::count_roots(P.I, t, w.forest(true), lo, hi, w.bits, w.counts, s, outside, true);
-  const ccl::Forest sel{w.R, nullptr, w.roots, w.nroots, nullptr};
+  const ccl::Forest sel{w.R, nullptr, w.roots, w.nroots};
   ccl::ZeroSpans z = call_spans(w, true, 0);
   z.n[1] = 0;  // the status holds the reconstruction's
   if (e == cudaSuccess) e = ccl::label(ClsValleyAbove{gt2}, P.I, t, 8, sel, s, z);
@@ -1526,10 +1225,7 @@ nsgb_status nsgb_imfill_holes(int dtype, const void* image, void* out, int64_t r
   }
   // Grayscale: erosion reconstruction of (image on the border, max inside) above the image.
   if (out == image) return NSGB_ERR_BAD_ARG;
-  dispatch_all(dtype, [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    e = fill_start<T>(dtype, P, w, (T*)out, conn, s);
-  });
+  e = fill_start_launch(dtype, P.I, P.t.c_tiles, w.forest(false), w.bits, w.bits_bytes, w.F, out, conn, s);
   if (e != cudaSuccess) return NSGB_ERR_CUDA;
   const Plan R = single_plan(dtype, out, image, rows, cols, pitch);
   // front from the border: re-sweep a tile up to four times when a neighbour changed while it
