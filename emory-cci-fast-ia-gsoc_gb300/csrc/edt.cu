@@ -16,19 +16,19 @@
 // is exact: no zero pixel further than 32 rows or columns away could be nearer.  Rows that hold a
 // pixel further away are marked and done again by the far pass.
 //   Bound: instructions issued (about 1.3 a pixel) beside the 5 bytes of a pixel.  4096^2 with
-//   objects of tens of pixels: 55 us (the far pass, which used to do every row: 179 us).
+//   objects of tens of pixels: 58 us (the far pass, which used to do every row: 179 us).
 //
 // Far pass, marked rows only (Meijster, Roerdink and Hesselink, 2000):
 // (1) per column, the distance in rows to the nearest zero pixel of that column, g (INF when the
-//     column has none; INF = rows + cols exceeds every real distance).  Columns are cut into
-//     128-row chunks: one launch records each chunk's first and last zero row, the next walks
-//     each chunk down and up from the nearest zero rows of the chunks above and below (threads
-//     of a warp take adjacent columns, so rows are read coalesced);
-// (2) per row, D^2(x) = min over x' of (x - x')^2 + g(x')^2, one CTA per row: each pixel
-//     searches outward along the row and stops once the column offset alone reaches its best
-//     squared distance (at most g(x) columns each way), which is cheap while the row's mean g is
-//     small.  A row with a large mean g (far from every zero pixel,
-//     or crossing columns without one) is done by the whole CTA by divide and conquer: the
+//     column has none; INF = rows + cols exceeds every real distance), from the same words.  Columns
+//     are cut into 128-row chunks: one launch records each chunk's first and last zero row, the next
+//     finds for each marked row the nearest zero rows within its word, its chunk or the chunks above
+//     and below (threads of a warp take adjacent columns, so g is written coalesced);
+// (2) per row, D^2(x) = min over x' of (x - x')^2 + g(x')^2, one CTA per row: each pixel that the
+//     near pass left searches outward along the row and stops once the column offset alone
+//     reaches its best squared distance (at most g(x) columns each way), which is cheap while the
+//     row's mean g is small.  A row with a large mean g (far from every zero pixel, or crossing
+//     columns without one) is done by the whole CTA by divide and conquer: the
 //     matrix (x - i)^2 + g(i)^2 is Monge, so the leftmost minimising column A(x) never
 //     decreases with x, and the row minimum at the midpoint of two computed positions a < b
 //     only needs the columns A(a) .. A(b).  Level by level (log2 W levels) every position's
@@ -44,46 +44,58 @@
 
 #include "common.cuh"
 #include "edt.cuh"
+#include "launch.cuh"
 
 namespace nsgb {
 
 namespace {
 
-constexpr int kThreads = 32;  // column passes: 32 adjacent columns per block
+constexpr int kThreads = 64;  // column passes: adjacent columns per block
 constexpr int kChunk = 128;   // rows per column chunk
 
 // ---- Near pass.
 
 constexpr int kNear = 32;       // rows of a tile and of a word; columns of halo on each side
 constexpr int kNearCols = 128;
-constexpr int kNearThreads = 256;
+// Threads of a near tile.  An image of few tiles leaves the device to their latency: there twice the
+// threads take half of the rows each (513 x 700 with far pixels all over: 9.9 -> 7.5 us).
+constexpr int kNearThreads = 256, kNearThreadsFew = 512, kNearFewTiles = 304;
 constexpr uint32_t kNearInf = 60000;  // a squared row distance beyond the near pass; + 32^2 < 2^16
 
 // Words of 32 rows: bit r of words[(y / 32) * W + x] is set where pixel (y + r, x) is zero.  Four
-// columns per thread; the four rows of a word's byte by byte: a byte's bits are eight rows.
+// columns per thread; the four rows of a word's byte by byte: a byte's bits are eight rows.  Clears the
+// marks of its rows on the way.
 template <bool VEC>
 __global__ void __launch_bounds__(128) edt_zero_words(const uint8_t* __restrict__ mask, int64_t pitch, int H, int W,
-                                                      uint32_t* __restrict__ words) {
+                                                      uint32_t* __restrict__ words, int* __restrict__ far,
+                                                      int* any_far) {
+  pdl_release();
   const int per = (W + 511) / 512, c = blockIdx.x / per;
+  if ((int)blockIdx.x == c * per && threadIdx.x < kNear && kNear * c + threadIdx.x < H) far[kNear * c + threadIdx.x] = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *any_far = 0;
   const int x = 4 * ((blockIdx.x - c * per) * blockDim.x + threadIdx.x);
   if (x >= W) return;
   const int y0 = kNear * c;
   const int last = H - 1 - y0;  // rows past the image repeat the last one; their bits are unused
-  uint32_t rows8[4];            // byte k: eight rows of column x + k
+  uint32_t px[kNear];           // all loads go out before the first is used
+#pragma unroll
+  for (int r = 0; r < kNear; ++r) {
+    const uint8_t* p = mask + (int64_t)(y0 + min(r, last)) * pitch + x;
+    if (VEC && x + 4 <= W) {
+      px[r] = __ldg((const uint32_t*)p);
+    } else {
+      px[r] = 0;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) px[r] |= (uint32_t)__ldg(p + min(b, W - 1 - x)) << (8 * b);
+    }
+  }
+  uint32_t rows8[4];  // byte k: eight rows of column x + k
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     uint32_t acc = 0;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
-      const uint8_t* p = mask + (int64_t)(y0 + min(8 * q + r, last)) * pitch + x;
-      uint32_t w;
-      if (VEC && x + 4 <= W) {
-        w = __ldg((const uint32_t*)p);
-      } else {
-        w = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) w |= (uint32_t)__ldg(p + min(b, W - 1 - x)) << (8 * b);
-      }
+      const uint32_t w = px[8 * q + r];
       // bit 7 of every zero byte
       const uint32_t z = ~(((w & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w) & 0x80808080u;
       acc |= z >> (7 - r);
@@ -107,16 +119,23 @@ __device__ __forceinline__ float near_value(uint32_t d2, bool basins) {
   return basins ? -d : d;
 }
 
-// Output of every pixel within 32 of a zero pixel; far[y] and *any_far where a row holds another.
-template <bool BASINS>
-__global__ void __launch_bounds__(kNearThreads) edt_near(const uint32_t* __restrict__ words, int nwords,
+// Output of every pixel within 32 of a zero pixel; where a row holds another, its bit in the row's far
+// words (W words apart), far[y] and *any_far.  (Marks are collected per CTA: stored by every pixel they were
+// 0.2 ms of a 4096^2 mask with most pixels far.)
+template <bool BASINS, int THREADS>
+__global__ void __launch_bounds__(THREADS) edt_near(const uint32_t* __restrict__ words, int nwords,
                                                          float* __restrict__ out, int64_t pitch_out, int H, int W,
-                                                         int* __restrict__ far, int* any_far) {
+                                                         uint32_t* __restrict__ far_words, int* __restrict__ far,
+                                                         int* any_far) {
+  pdl_wait();
+  pdl_release();
   constexpr int kCols = kNearCols + 2 * kNear;
   __shared__ uint32_t s[kNear / 2][kCols];  // rows 2 j (low half) and 2 j + 1 (high half), squared
+  __shared__ int s_far[kNear];
   const int per = (W + kNearCols - 1) / kNearCols, c = blockIdx.x / per;
   const int x0 = (blockIdx.x - c * per) * kNearCols, y0 = c * kNear;
   bool seen = false;
+  if (threadIdx.x < kNear) s_far[threadIdx.x] = 0;
   if (threadIdx.x < kCols) {
     const int x = x0 - kNear + threadIdx.x;
     uint32_t z = 0, above = 0, below = 0;
@@ -146,10 +165,13 @@ __global__ void __launch_bounds__(kNearThreads) edt_near(const uint32_t* __restr
   if (!__syncthreads_or(seen)) {  // no zero pixel anywhere near
     if (threadIdx.x < kNear && y0 + threadIdx.x < H) far[y0 + threadIdx.x] = 1;
     if (threadIdx.x == 0) *any_far = 1;
+    constexpr int kWords = kNearCols / 32;
+    const int y = y0 + threadIdx.x / kWords, x = x0 + 32 * (threadIdx.x % kWords);
+    if (threadIdx.x < kNear * kWords && y < H && x < W) far_words[(int64_t)y * W + x / 32] = 0xFFFFFFFFu;
     return;
   }
   const int x = x0 + (threadIdx.x & (kNearCols - 1));
-  for (int j = threadIdx.x / kNearCols; j < kNear / 2; j += kNearThreads / kNearCols) {
+  for (int j = threadIdx.x / kNearCols; j < kNear / 2; j += THREADS / kNearCols) {  // the same for a warp
     const int y = y0 + 2 * j;
     if (y >= H) break;
     const uint32_t* row = s[j] + kNear + (threadIdx.x & (kNearCols - 1));
@@ -162,68 +184,140 @@ __global__ void __launch_bounds__(kNearThreads) edt_near(const uint32_t* __restr
         best = __vimin3_u16x2(best, row[-(k + q)] + kk, row[k + q] + kk);
       }
     }
-    if (x >= W) continue;
-    const uint32_t lo = best & 0xFFFFu, hi = best >> 16;
-    float* o = (float*)((char*)out + (int64_t)y * pitch_out) + x;
-    if (lo <= kNear * kNear) *o = near_value(lo, BASINS);
-    else far[y] = *any_far = 1;
-    if (y + 1 < H) {
-      if (hi <= kNear * kNear) *(float*)((char*)o + pitch_out) = near_value(hi, BASINS);
-      else far[y + 1] = *any_far = 1;
+    const uint32_t d[2] = {best & 0xFFFFu, best >> 16};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (y + h >= H) break;
+      const bool in = x < W, is_far = d[h] > kNear * kNear;
+      if (in && !is_far) *((float*)((char*)out + (int64_t)(y + h) * pitch_out) + x) = near_value(d[h], BASINS);
+      const unsigned word = __ballot_sync(NSGB_FULL, in && is_far);
+      if ((threadIdx.x & 31) == 0 && in) {
+        far_words[(int64_t)(y + h) * W + x / 32] = word;
+        if (word) s_far[2 * j + h] = 1;
+      }
     }
+  }
+  __syncthreads();
+  if (threadIdx.x < kNear) {
+    const bool mark = s_far[threadIdx.x] != 0;
+    if (mark) far[y0 + threadIdx.x] = 1;
+    if (__any_sync(NSGB_FULL, mark) && threadIdx.x == 0) *any_far = 1;
   }
 }
 
 // ---- Far pass.
 
+constexpr int kChunkWords = kChunk / kNear;
+
 // First and last zero row of every (column, chunk), -1 when none.
-__global__ void __launch_bounds__(kThreads) edt_chunk_zeros(const uint8_t* __restrict__ mask, int64_t pitch, int H,
-                                                            int W, int* __restrict__ first0, int* __restrict__ last0,
+__global__ void __launch_bounds__(kThreads) edt_chunk_zeros(const uint32_t* __restrict__ words, int nwords, int W,
+                                                            int* __restrict__ first0, int* __restrict__ last0,
                                                             const int* __restrict__ any_far) {
+  pdl_wait();
+  pdl_release();
   if (*any_far == 0) return;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= W) return;
   const int c = blockIdx.y;
-  const int y0 = c * kChunk, y1 = min(H, y0 + kChunk);
   int f = -1, l = -1;
-  for (int y = y0; y < y1; ++y)
-    if (__ldg(mask + (int64_t)y * pitch + x) == 0) {
-      if (f < 0) f = y;
-      l = y;
+#pragma unroll
+  for (int q = 0; q < kChunkWords; ++q) {
+    const int k = c * kChunkWords + q;
+    const uint32_t w = k < nwords ? __ldg(words + (int64_t)k * W + x) : 0u;
+    if (w) {
+      if (f < 0) f = k * kNear + __ffs(w) - 1;
+      l = k * kNear + 31 - __clz(w);
     }
+  }
   first0[(int64_t)c * W + x] = f;
   last0[(int64_t)c * W + x] = l;
 }
 
-// g for the rows of one (column, chunk): nearest zero row above (from the chunks above, then
-// this chunk's rows in order) and below.
-__global__ void __launch_bounds__(kThreads) edt_columns(const uint8_t* __restrict__ mask, int64_t pitch, int H, int W,
+// g of one row, `up` and `down` its column's zero pixels of the word at or above and at or below the row.
+__device__ __forceinline__ int row_distance(uint32_t up, uint32_t down, int y, int above, int below, int inf) {
+  const int du = up ? __clz(up) : above >= 0 ? y - above : inf;
+  const int dd = down ? __ffs(down) - 1 : below >= 0 ? below - y : inf;
+  return min(du, dd);
+}
+
+// g for the marked rows of one (column, chunk), from the words of zero pixels: nearest zero row above and
+// below, in the chunk or in the chunks above and below it.  (Walked pixel by pixel down and up, with g
+// written, read and written again, this pass took 59 us at 4096^2, and the one before it another 16 MB of
+// mask.)
+__global__ void __launch_bounds__(kThreads) edt_columns(const uint32_t* __restrict__ words, int nwords, int H, int W,
                                                         const int* __restrict__ first0, const int* __restrict__ last0,
                                                         int* __restrict__ g, const int* __restrict__ far,
                                                         const int* __restrict__ any_far) {
+  pdl_wait();
+  pdl_release();
   if (*any_far == 0) return;
-  const int c = blockIdx.y, nc = gridDim.y;
-  const int y0 = c * kChunk, y1 = min(H, y0 + kChunk);
-  int marked = 0;  // rows of this chunk that the far pass does
-  for (int y = y0 + threadIdx.x; y < y1; y += kThreads) marked |= __ldg(far + y);
-  if (!__any_sync(NSGB_FULL, marked)) return;
+  const int c = blockIdx.y, nc = gridDim.y, lane = threadIdx.x & 31;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= W) return;
-  const int inf = H + W;
-  int z = -1;  // nearest zero row at or above the current row
-  for (int k = c - 1; k >= 0 && z < 0; --k) z = __ldg(last0 + (int64_t)k * W + x);
-  for (int y = y0; y < y1; ++y) {
-    if (__ldg(mask + (int64_t)y * pitch + x) == 0) z = y;
-    g[(int64_t)y * W + x] = z >= 0 ? y - z : inf;
+  uint32_t marked[kChunkWords];  // rows of this chunk that the far pass does
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < kChunkWords; ++q) {
+    const int y = c * kChunk + q * kNear + lane;
+    marked[q] = __ballot_sync(NSGB_FULL, y < H && __ldg(far + (y < H ? y : 0)) != 0);
+    any = any || marked[q] != 0u;
   }
-  z = -1;  // nearest zero row at or below
-  for (int k = c + 1; k < nc && z < 0; ++k) z = __ldg(first0 + (int64_t)k * W + x);
-  for (int y = y1 - 1; y >= y0; --y) {
-    if (__ldg(mask + (int64_t)y * pitch + x) == 0) z = y;
-    if (z >= 0) {
-      int* p = g + (int64_t)y * W + x;
-      if (z - y < *p) *p = z - y;
+  if (!any || x >= W) return;
+  const int inf = H + W;
+  int above = -1, below = -1;  // nearest zero rows outside the chunk
+  for (int k = c - 1; k >= 0 && above < 0; --k) above = __ldg(last0 + (int64_t)k * W + x);
+  for (int k = c + 1; k < nc && below < 0; ++k) below = __ldg(first0 + (int64_t)k * W + x);
+  uint32_t w[kChunkWords];
+#pragma unroll
+  for (int q = 0; q < kChunkWords; ++q) {
+    const int k = c * kChunkWords + q;
+    w[q] = k < nwords ? __ldg(words + (int64_t)k * W + x) : 0u;
+  }
+#pragma unroll
+  for (int q = 0; q < kChunkWords; ++q) {
+    const int y0 = c * kChunk + q * kNear;
+    if (marked[q]) {
+      int next = below;  // nearest zero row below the word
+#pragma unroll
+      for (int p = kChunkWords - 1; p > q; --p)
+        if (w[p]) next = c * kChunk + p * kNear + __ffs(w[p]) - 1;
+#pragma unroll 8
+      for (int r = 0; r < kNear; ++r) {
+        if (!((marked[q] >> r) & 1u)) continue;  // the same for a warp
+        g[(int64_t)(y0 + r) * W + x] = row_distance(w[q] << (31 - r), w[q] >> r, y0 + r, above, next, inf);
+      }
     }
+    if (w[q]) above = y0 + 31 - __clz(w[q]);
+  }
+}
+
+// The same in one launch for images of up to kFewWords words of rows: a thread per (column, word) loads the
+// column's words, all at once.  A short image leaves the device to the latency of the two launches above,
+// each of few CTAs (513 x 700: 15 us of chunks and columns, this 6).
+constexpr int kFewWords = 32;
+__global__ void __launch_bounds__(kThreads) edt_columns_few(const uint32_t* __restrict__ words, int nwords, int H, int W,
+                                                            int* __restrict__ g, const int* __restrict__ far,
+                                                            const int* __restrict__ any_far) {
+  pdl_wait();
+  pdl_release();
+  if (*any_far == 0) return;
+  const int c = blockIdx.y, y0 = c * kNear, lane = threadIdx.x & 31;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, xc = min(x, W - 1);
+  uint32_t w[kFewWords];
+#pragma unroll
+  for (int k = 0; k < kFewWords; ++k) w[k] = k < nwords ? __ldg(words + (int64_t)k * W + xc) : 0u;
+  const uint32_t marked = __ballot_sync(NSGB_FULL, y0 + lane < H && __ldg(far + min(y0 + lane, H - 1)) != 0);
+  if (!marked || x >= W) return;
+  int above = -1, below = -1;
+  uint32_t own = 0u;
+#pragma unroll
+  for (int k = 0; k < kFewWords; ++k) {
+    if (k < c && w[k]) above = k * kNear + 31 - __clz(w[k]);
+    if (k == c) own = w[k];
+    if (k > c && w[k] && below < 0) below = k * kNear + __ffs(w[k]) - 1;
+  }
+  for (uint32_t m = marked; m; m &= m - 1u) {
+    const int r = __ffs(m) - 1;
+    g[(int64_t)(y0 + r) * W + x] = row_distance(own << (31 - r), own >> r, y0 + r, above, below, H + W);
   }
 }
 
@@ -404,9 +498,10 @@ __device__ void dc_row(const int* __restrict__ gr, float* o, const uint8_t* mrow
 template <bool BASINS>
 __global__ void __launch_bounds__(kRowThreads) edt_rows(const uint8_t* __restrict__ mask, int64_t pitch_in,
                                                         const int* __restrict__ g, int* __restrict__ stack_s,
-                                                        int* __restrict__ stack_t, float* __restrict__ out,
+                                                        int* stack_t, float* __restrict__ out,
                                                         int64_t pitch_out, int H, int W, bool dc,
                                                         const int* __restrict__ far, const int* __restrict__ any_far) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char dc_smem[];
   __shared__ long long s_sum[kRowThreads / 32];
   if (*any_far == 0) return;
@@ -425,7 +520,9 @@ __global__ void __launch_bounds__(kRowThreads) edt_rows(const uint8_t* __restric
 #pragma unroll
     for (int k = 0; k < kRowThreads / 32; ++k) total += s_sum[k];
     if (total <= kMeanG * W) {
+      const int* far_word = stack_t + (int64_t)y * W;  // the near pass's: the other pixels are done
       for (int x = threadIdx.x; x < W; x += kRowThreads) {
+        if (!((__ldg(far_word + x / 32) >> (x & 31)) & 1)) continue;
         const int64_t gx = __ldg(gr + x);
         int64_t best = gx * gx;
         for (int64_t k = 1; k < W && k * k < best; ++k) {
@@ -467,40 +564,47 @@ cudaError_t edt_launch(const uint8_t* mask, int64_t pitch_in, float* out, int64_
   uint32_t* words = (uint32_t*)st_s;
   int* any_far = (int*)(p + 3 * plane + 2 * chunks);
   int* far = any_far + 64;
-  cudaError_t e = cudaMemsetAsync(any_far, 0, 256 + sizeof(int) * (size_t)rows, s);
-  if (e != cudaSuccess) return e;
+  // The far words lie in each row's part of the other stack plane: a row takes either them or the stacks.
+  uint32_t* far_words = (uint32_t*)st_t;
+  cudaError_t e = cudaSuccess;
   const unsigned wgrid = (unsigned)nwords * (unsigned)((cols + 511) / 512);
   const unsigned ngrid = (unsigned)nwords * (unsigned)((cols + kNearCols - 1) / kNearCols);
+  const bool few = ngrid <= kNearFewTiles;
   if ((uintptr_t)mask % 4 == 0 && pitch_in % 4 == 0)
-    edt_zero_words<true><<<wgrid, 128, 0, s>>>(mask, pitch_in, rows, cols, words);
+    edt_zero_words<true><<<wgrid, 128, 0, s>>>(mask, pitch_in, rows, cols, words, far, any_far);
   else
-    edt_zero_words<false><<<wgrid, 128, 0, s>>>(mask, pitch_in, rows, cols, words);
-  if (basins)
-    edt_near<true><<<ngrid, kNearThreads, 0, s>>>(words, nwords, out, pitch_out, rows, cols, far, any_far);
-  else
-    edt_near<false><<<ngrid, kNearThreads, 0, s>>>(words, nwords, out, pitch_out, rows, cols, far, any_far);
+    edt_zero_words<false><<<wgrid, 128, 0, s>>>(mask, pitch_in, rows, cols, words, far, any_far);
+  e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = launch_dependent(few ? (basins ? edt_near<true, kNearThreadsFew> : edt_near<false, kNearThreadsFew>)
+                             : (basins ? edt_near<true, kNearThreads> : edt_near<false, kNearThreads>),
+                         dim3(ngrid), dim3(few ? kNearThreadsFew : kNearThreads), s, (const uint32_t*)words, nwords, out, pitch_out, rows, cols, far_words, far, any_far);
   const dim3 cgrid((cols + kThreads - 1) / kThreads, nchunks);
-  edt_chunk_zeros<<<cgrid, kThreads, 0, s>>>(mask, pitch_in, rows, cols, first0, last0, any_far);
-  edt_columns<<<cgrid, kThreads, 0, s>>>(mask, pitch_in, rows, cols, first0, last0, g, far, any_far);
+  if (nwords <= kFewWords) {
+    if (e == cudaSuccess)
+      e = launch_dependent(edt_columns_few, dim3(cgrid.x, nwords), dim3(kThreads), s, (const uint32_t*)words, nwords, rows,
+                           cols, g, (const int*)far, (const int*)any_far);
+  } else {
+    if (e == cudaSuccess)
+      e = launch_dependent(edt_chunk_zeros, cgrid, dim3(kThreads), s, (const uint32_t*)words, nwords, cols, first0,
+                           last0, (const int*)any_far);
+    if (e == cudaSuccess)
+      e = launch_dependent(edt_columns, cgrid, dim3(kThreads), s, (const uint32_t*)words, nwords, rows, cols,
+                           (const int*)first0, (const int*)last0, g, (const int*)far, (const int*)any_far);
+  }
   const int rblocks = rows < (1 << 20) ? rows : (1 << 20);
   // divide and conquer: tables fit (u16 columns, 24-bit column field) and 2 (H + W)^2 < 2^40
   const bool dc = cols <= kDcMaxW && (int64_t)rows + cols < (1 << 19);
   const size_t smem = dc ? (((size_t)cols * 2 + 15) & ~(size_t)15) + (size_t)(cols / 2 + 1) * 8 +
                                (size_t)(cols / 2 + 2) * 4
                          : 0;
-  if (basins) {
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(edt_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      edt_rows<true><<<rblocks, kRowThreads, smem, s>>>(mask, pitch_in, g, st_s, st_t, out, pitch_out, rows, cols, dc,
-                                                      far, any_far);
-  } else {
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(edt_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      edt_rows<false><<<rblocks, kRowThreads, smem, s>>>(mask, pitch_in, g, st_s, st_t, out, pitch_out, rows, cols, dc,
-                                                      far, any_far);
-  }
-  if (e != cudaSuccess) return e;
-  return cudaGetLastError();
+  const auto rows_kernel = basins ? edt_rows<true> : edt_rows<false>;
+  if (e == cudaSuccess && smem > 48 * 1024)
+    e = cudaFuncSetAttribute(rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess)
+    e = launch_dependent_smem(rows_kernel, dim3(rblocks), dim3(kRowThreads), smem, s, mask, pitch_in, (const int*)g, st_s,
+                              st_t, out, pitch_out, rows, cols, dc, (const int*)far, (const int*)any_far);
+  return e;
 }
 
 }  // namespace nsgb
