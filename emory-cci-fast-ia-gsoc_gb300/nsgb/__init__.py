@@ -58,52 +58,45 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+class _Buffer:
+    """One cached workspace, a uint8 tensor grown on demand; `get` under `lock` only."""
+
+    __slots__ = ("lock", "device", "_tensor", "_at", "_size")
+
+    def __init__(self, device: torch.device) -> None:
+        self.lock = threading.RLock()
+        self.device, self._tensor, self._at, self._size = device, None, 0, 0
+
+    def get(self, nbytes: int) -> Tuple[int, int]:
+        if self._size < nbytes:
+            t = torch.empty(max(nbytes, 1 << 20) + 256, dtype=torch.uint8, device=self.device)
+            # the next holder may run on another stream than the one this memory comes from
+            torch.cuda.current_stream(self.device).synchronize()
+            at = (t.data_ptr() + 255) & ~255
+            self._tensor, self._at, self._size = t, at, t.numel() - (at - t.data_ptr())
+        return self._at, self._size
+
+
 class _Workspace:
-    """Cached workspaces (uint8 tensors grown on demand), one per key: the device, and the direction
-    for the float pair.  A call holds its buffer from the size lookup until it has returned, by when its
-    kernels are done: the library runs without the GIL, so calls of several threads would otherwise
-    run on one status word, tile queue and label forest at once."""
+    """Cached workspaces, one per device (and one per direction of the float pair).  A call holds its
+    buffer's lock from the size lookup until it has returned, by when its kernels are done: the library
+    runs without the GIL, so calls of several threads would otherwise run on one status word, tile
+    queue and label forest at once."""
 
     def __init__(self) -> None:
-        self._buf: Dict[object, torch.Tensor] = {}
-        self._locks: Dict[object, threading.RLock] = {}
+        self._buffers: Dict[object, _Buffer] = {}
 
-    def get(self, nbytes: int, device: torch.device, key: object = None) -> Tuple[int, int]:
-        if key is None:
-            key = device.index if device.index is not None else torch.cuda.current_device()
-        buf = self._buf.get(key)
-        if buf is None or buf.numel() < nbytes:
-            buf = torch.empty(max(nbytes, 1 << 20) + 256, dtype=torch.uint8, device=device)
-            # the next holder may run on another stream than the one this memory comes from
-            torch.cuda.current_stream(device).synchronize()
-            self._buf[key] = buf
-        ptr = buf.data_ptr()
-        aligned = (ptr + 255) & ~255
-        return aligned, buf.numel() - (aligned - ptr)
+    def buffer(self, device: torch.device, kind: str = "") -> _Buffer:
+        key = (device, kind)
+        b = self._buffers.get(key)
+        return b if b is not None else self._buffers.setdefault(key, _Buffer(device))
 
-    def hold(self, nbytes: int, device: torch.device, kind: str = "") -> "_Held":
-        """The buffer for a `with` block: (address, bytes), for this thread alone."""
-        idx = device.index if device.index is not None else torch.cuda.current_device()
-        key = (idx, kind) if kind else idx
-        return _Held(self, self._locks.setdefault(key, threading.RLock()), nbytes, device, key)
-
-
-class _Held:
-    __slots__ = ("pool", "lock", "nbytes", "device", "key")
-
-    def __init__(self, pool, lock, nbytes, device, key) -> None:
-        self.pool, self.lock, self.nbytes, self.device, self.key = pool, lock, nbytes, device, key
-
-    def __enter__(self) -> Tuple[int, int]:
-        self.lock.acquire()
-        try:
-            return self.pool.get(self.nbytes, self.device, self.key)
-        except BaseException:
-            self.lock.release()
-            raise
-
-    def __exit__(self, *exc) -> None:
-        self.lock.release()
+    def get(self, nbytes: int, device: torch.device) -> Tuple[int, int]:
+        if device.index is None:
+            device = torch.device(device.type, torch.cuda.current_device())
+        b = self.buffer(device)
+        with b.lock:
+            return b.get(nbytes)
 
 
 workspace = _Workspace()
@@ -112,8 +105,8 @@ workspace = _Workspace()
 _workspace_size = functools.lru_cache(maxsize=256)(lib.nsgb_workspace_size)
 
 
-def _ws(op: int, dtype: int, rows: int, cols: int, device: torch.device) -> _Held:
-    return workspace.hold(_workspace_size(op, dtype, rows, cols), device)
+def _ws(op: int, dtype: int, rows: int, cols: int, device: torch.device) -> Tuple[_Buffer, int]:
+    return workspace.buffer(device), _workspace_size(op, dtype, rows, cols)
 
 
 def _same_shape(a: torch.Tensor, b: torch.Tensor, what: str) -> None:
@@ -144,7 +137,9 @@ def imreconstruct(seeds: torch.Tensor, image: torch.Tensor, connectivity: int, e
     mask = _contig(image)
     rows, cols = out.shape
     opts = _ffi.Opts(1, max_visits_per_tile, max_visit_iters, queue_poll_limit)
-    with _ws(_ffi.OP_IMRECONSTRUCT, dt, rows, cols, out.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_IMRECONSTRUCT, dt, rows, cols, out.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_imreconstruct(dt, out.data_ptr(), mask.data_ptr(), rows, cols, _pitch(out), connectivity,
                                     1 if erode else 0, ws, nb, _stream(), C.byref(opts))
     _ffi.check(st, "imreconstruct")
@@ -160,7 +155,9 @@ def imreconstructBinary(seeds: torch.Tensor, binaryImage: torch.Tensor, connecti
     out = _contig(seeds).clone()
     mask = _contig(binaryImage)
     rows, cols = out.shape
-    with _ws(_ffi.OP_IMRECONSTRUCT_BINARY, dt, rows, cols, out.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_IMRECONSTRUCT_BINARY, dt, rows, cols, out.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_imreconstruct_binary(dt, out.data_ptr(), mask.data_ptr(), rows, cols, _pitch(out), connectivity,
                                            ws, nb, _stream(), None)
     _ffi.check(st, "imreconstructBinary")
@@ -174,7 +171,9 @@ def imfillHoles(image: torch.Tensor, binary: bool, connectivity: int) -> torch.T
     img = _contig(image)
     out = _dense_like(img)
     rows, cols = img.shape
-    with _ws(_ffi.OP_FILL_HOLES, dt, rows, cols, img.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_FILL_HOLES, dt, rows, cols, img.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_imfill_holes(dt, img.data_ptr(), out.data_ptr(), rows, cols, _pitch(img), 1 if binary else 0,
                                    connectivity, ws, nb, _stream(), None)
     _ffi.check(st, "imfillHoles")
@@ -188,7 +187,9 @@ def imhmin(image: torch.Tensor, h: float, connectivity: int) -> torch.Tensor:
     img = _contig(image)
     out = _dense_like(img)
     rows, cols = img.shape
-    with _ws(_ffi.OP_HMIN, dt, rows, cols, img.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_HMIN, dt, rows, cols, img.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_imhmin(dt, img.data_ptr(), out.data_ptr(), rows, cols, _pitch(img), float(h), connectivity, ws,
                              nb, _stream(), None)
     _ffi.check(st, "imhmin")
@@ -205,7 +206,9 @@ def bwselect(binaryImage: torch.Tensor, seeds: torch.Tensor, connectivity: int) 
     sd = _contig(seeds)
     out = _dense_like(img)
     rows, cols = img.shape
-    with _ws(_ffi.OP_BWSELECT, dt, rows, cols, img.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_BWSELECT, dt, rows, cols, img.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_bwselect(dt, img.data_ptr(), sd.data_ptr(), out.data_ptr(), rows, cols, _pitch(img), connectivity,
                                ws, nb, _stream(), None)
     _ffi.check(st, "bwselect")
@@ -233,7 +236,9 @@ def _bwlabel(binaryImage: torch.Tensor, connectivity: int, relab: bool) -> Tuple
     rows, cols = img.shape
     lab = torch.empty((rows, cols), dtype=torch.int32, device=img.device)
     n = C.c_int32(0)
-    with _ws(_ffi.OP_BWLABEL, _ffi.U8, rows, cols, img.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_BWLABEL, _ffi.U8, rows, cols, img.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_bwlabel(img.data_ptr(), lab.data_ptr(), rows, cols, _pitch(img), _pitch(lab), connectivity,
                               1 if relab else 0, C.byref(n), ws, nb, _stream(), None)
     _ffi.check(st, "bwlabel2")
@@ -259,7 +264,9 @@ def bwareaopen2(image: torch.Tensor, labeled: bool, flatten: bool, minSize: int,
     img = _contig(image)
     rows, cols = img.shape
     cnt = C.c_int32(0)
-    with _ws(_ffi.OP_BWAREAOPEN, _ffi.U8, rows, cols, img.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_BWAREAOPEN, _ffi.U8, rows, cols, img.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         if flatten:
             out = torch.empty((rows, cols), dtype=torch.uint8, device=img.device)
             st = lib.nsgb_bwareaopen(img.data_ptr(), 1 if labeled else 0, None, out.data_ptr(), rows, cols, _pitch(img),
@@ -287,12 +294,13 @@ def bounding_boxes(labels: torch.Tensor, bgval: int = 0, capacity: Optional[int]
         raise NsgbError(2, "labels must be int32")
     lab = _contig(labels)
     rows, cols = lab.shape
-    hold = _ws(_ffi.OP_BOUNDING_BOX, _ffi.I32, rows, cols, lab.device)
+    buf, need = _ws(_ffi.OP_BOUNDING_BOX, _ffi.I32, rows, cols, lab.device)
     cap = min(rows * cols, 65536 if capacity is None else max(1, int(capacity)))
     while True:
         boxes = torch.empty((5, cap), dtype=torch.int32, device=lab.device)
         cnt = C.c_int32(0)
-        with hold as (ws, nb):
+        with buf.lock:
+            ws, nb = buf.get(need)
             st = lib.nsgb_bounding_boxes(lab.data_ptr(), rows, cols, _pitch(lab), int(bgval), boxes.data_ptr(), cap,
                                          C.byref(cnt), None, ws, nb, _stream(), None)
         _ffi.check(st, "bounding_boxes")
@@ -342,7 +350,9 @@ def chain(marker: torch.Tensor, mask: torch.Tensor, recon_conn: int = 8, thr: fl
     labels = torch.empty((rows, cols), dtype=torch.int32, device=dev)
     area = torch.empty((rows, cols), dtype=torch.uint8, device=dev)
     nl, nk = C.c_int32(0), C.c_int32(0)
-    with _ws(_ffi.OP_CHAIN, dt, rows, cols, dev) as (ws, nb):
+    buf, need = _ws(_ffi.OP_CHAIN, dt, rows, cols, dev)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_chain(dt, rec.data_ptr(), msk.data_ptr(), rows, cols, _pitch(rec), recon_conn, float(thr),
                             fill_conn, label_conn, int(area_min), int(area_max), fill.data_ptr(), labels.data_ptr(),
                             area.data_ptr(), C.byref(nl), C.byref(nk), ws, nb, _stream(), None)
@@ -386,7 +396,9 @@ def morphOpen(image: torch.Tensor, kernel) -> torch.Tensor:
     img = _contig(image)
     rows, cols = img.shape
     out = torch.empty((rows, cols), dtype=torch.uint8, device=img.device)
-    with _ws(_ffi.OP_MORPH_OPEN, _ffi.U8, rows, cols, img.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_MORPH_OPEN, _ffi.U8, rows, cols, img.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_morph_open(img.data_ptr(), out.data_ptr(), rows, cols, _pitch(img), _pitch(out),
                                  k.ctypes.data_as(C.c_void_p), int(k.shape[0]), ws, nb, _stream(), None)
     _ffi.check(st, "morphOpen")
@@ -404,7 +416,9 @@ def distanceTransform(mask: torch.Tensor, basins: bool = False) -> torch.Tensor:
     m = _contig(mask)
     rows, cols = m.shape
     out = torch.empty((rows, cols), dtype=torch.float32, device=m.device)
-    with _ws(_ffi.OP_DISTANCE, _ffi.U8, rows, cols, m.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_DISTANCE, _ffi.U8, rows, cols, m.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_distance_transform(m.data_ptr(), out.data_ptr(), rows, cols, _pitch(m), _pitch(out),
                                          1 if basins else 0, ws, nb, _stream(), None)
     _ffi.check(st, "distanceTransform")
@@ -429,7 +443,9 @@ def nucleus_candidates(rc: torch.Tensor, rc_open: torch.Tensor, rbc: torch.Tenso
     rows, cols = rec.shape
     seg = torch.empty((rows, cols), dtype=torch.uint8, device=rec.device)
     nk = C.c_int32(0)
-    with _ws(_ffi.OP_NUCLEUS_CANDIDATES, _ffi.U8, rows, cols, rec.device) as (ws, nb):
+    buf, need = _ws(_ffi.OP_NUCLEUS_CANDIDATES, _ffi.U8, rows, cols, rec.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_nucleus_candidates(rec.data_ptr(), img.data_ptr(), red.data_ptr(), seg.data_ptr(), rows, cols,
                                          _pitch(rec), float(g1), float(g2), int(area_min), int(area_max), C.byref(nk),
                                          None, ws, nb, _stream(), None)
@@ -534,11 +550,11 @@ def _stack3(t: torch.Tensor, name: str) -> torch.Tensor:
     return t if t.dim() == 3 else t.unsqueeze(0)
 
 
-def _f32_workspace(B, H, W, backward, dev) -> _Held:
+def _f32_workspace(B, H, W, backward, dev) -> Tuple[_Buffer, int]:
     need = lib.nsgb_recon_f32_workspace_size(B, H, W, 1 if backward else 0)
     if need == 0:
         raise NsgbError(1, "recon_f32: image stack too large")
-    return workspace.hold(need, dev, "f32 backward" if backward else "f32 forward")
+    return workspace.buffer(dev, "f32 backward" if backward else "f32 forward"), need
 
 
 def recon_f32(marker: torch.Tensor, mask: torch.Tensor, connectivity: int = 8):
@@ -551,7 +567,9 @@ def recon_f32(marker: torch.Tensor, mask: torch.Tensor, connectivity: int = 8):
     B, H, W = ms.shape
     out = torch.empty_like(ms)
     prov = torch.empty(ms.shape, dtype=torch.int32, device=ms.device)
-    with _f32_workspace(B, H, W, False, ms.device) as (ws, nb):
+    buf, need = _f32_workspace(B, H, W, False, ms.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_recon_f32_fwd(mk.data_ptr(), ms.data_ptr(), out.data_ptr(), prov.data_ptr(), B, H, W, W * 4,
                                     H * W * 4, connectivity, ws, nb, _stream(), None)
     _ffi.check(st, "recon_f32_fwd")
@@ -569,7 +587,9 @@ def recon_f32_backward(grad: torch.Tensor, prov: torch.Tensor):
     B, H, W = g.shape
     dm = torch.empty_like(g)
     dk = torch.empty_like(g)
-    with _f32_workspace(B, H, W, True, g.device) as (ws, nb):
+    buf, need = _f32_workspace(B, H, W, True, g.device)
+    with buf.lock:
+        ws, nb = buf.get(need)
         st = lib.nsgb_recon_f32_bwd(g.data_ptr(), p.data_ptr(), dm.data_ptr(), dk.data_ptr(), B, H, W, W * 4,
                                     H * W * 4, ws, nb, _stream(), None)
     _ffi.check(st, "recon_f32_bwd")
