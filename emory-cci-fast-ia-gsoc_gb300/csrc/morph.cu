@@ -6,7 +6,7 @@
 // not reflected for the dilation); pixels outside the image read the padding value.
 //
 // One CTA computes a 128-row x 128-column output tile, four pixels to a 32-bit word, one word
-// column per lane, eight rows per warp.  The input rows the tile needs (64 + 2 bw, with 32 columns
+// column per lane, eight rows per warp.  The input rows the tile needs (128 + 2 bw, with 32 columns
 // of halo on each side) are staged in shared memory once, padding values filled in; the word at
 // any column offset is one funnel shift of two staged words.
 //
@@ -24,7 +24,7 @@
 // one per plane, between two barriers), and the element rows of that radius fold the plane's rows
 // into the per-row accumulators.  A vertical run of eight or more element rows of one radius is a
 // sliding window: the rows common to a thread's eight outputs are folded once.
-// Other elements take the direct path: one fold per element pixel.
+// Other elements take the direct path: two folds (odd and even pixels) per element pixel.
 //
 // Bound: instructions issued.  4096^2 with the 19 x 19 disk: 49 us per pass at 66% of
 // issue cycles (the byte-wise form, one radius per barrier pair and 64-row tiles, took 102 us; this
@@ -68,12 +68,6 @@ __device__ __forceinline__ void fold_quad(Quad& a, uint32_t w) {
   a.even = fold<MAX>(a.even, w << 8);
 }
 __device__ __forceinline__ uint32_t pixels(const Quad& q) { return __byte_perm(q.even, q.odd, 0x7351); }
-
-// The four pixels starting `s` columns right of word column `cw` of a staged row.
-__device__ __forceinline__ uint32_t word_at(const uint32_t* row, int cw, int s) {
-  const int pos = 4 * (kHaloWords + cw) + s;
-  return __funnelshift_r(row[pos >> 2], row[(pos >> 2) + 1], 8 * (pos & 3));
-}
 
 // The element rows of radius r, from their plane, into the eight outputs of this thread (tile
 // rows j0 ..; element row i of output j is plane row j + i).
@@ -124,9 +118,10 @@ __device__ __forceinline__ void fold_rows(Quad (&acc)[kRowsPerWarp], const uint3
   }
 }
 
-// MAX = false: erosion, padding 255; MAX = true: dilation, padding 0.  Dynamic shared memory:
-// morph_smem(bw) bytes.
-template <bool MAX>
+// MAX = false: erosion, padding 255; MAX = true: dilation, padding 0.  CENTRED: the fast path (a kernel of
+// its own: fetched cold, one with both paths took 5 us longer a pass).  Dynamic shared memory:
+// morph_smem(e) bytes.
+template <bool MAX, bool CENTRED>
 __global__ void __launch_bounds__(kThreads, 2) morph_kernel(const uint8_t* __restrict__ in, int64_t pitch_in,
                                                          bool in_words, bool in_quads, uint8_t* __restrict__ out,
                                                          int64_t pitch_out, bool out_words, int H, int W,
@@ -189,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 2) morph_kernel(const uint8_t* __res
     for (int j = 0; j < kRowsPerWarp; ++j) acc[j] = Quad{pad, pad};
     const int j0 = warp * kRowsPerWarp;  // this warp's first output row in the tile
 
-    if (e.centred) {
+    if constexpr (CENTRED) {
       // radius 0: the staged rows themselves
       if (e.radii & 1u) {
         for (int i = warp; i < rows_in; i += kWarps) R[i * kTileWords + lane] = S[i * kRowWords + kHaloWords + lane];
@@ -247,16 +242,45 @@ __global__ void __launch_bounds__(kThreads, 2) morph_kernel(const uint8_t* __res
         __syncthreads();
       }
     } else {
+      // Any element, row by row: each word that a row's columns reach is loaded once for the eight outputs,
+      // and the word at each used column offset formed once, for the odd pixels at that offset and the
+      // even ones at the next (a word formed anew for each element pixel and parity took 2.0 ms for an opening
+      // of 4096^2 by a random 19 x 19 element, 0.55 now).
+      const int wd0 = -((e.bw + 4) / 4);  // the word of offset -bw - 1, below
       for (int kr = 0; kr < e.k; ++kr) {
-        const uint64_t bits = e.row_bits[kr];
+        const uint64_t bits = e.row_bits[kr];  // bit i: offset i - bw for odd pixels, i - bw - 1 for even ones
         if (!bits) continue;
+        const uint32_t* row = S + (j0 + kr) * kRowWords + kHaloWords + lane;
+        uint32_t cur[kRowsPerWarp], next[kRowsPerWarp];
+        bool loaded = false;  // next holds the word that becomes cur
+        for (int wd = wd0; 4 * wd <= e.bw; ++wd) {
+          const int i0 = 4 * wd + e.bw + 1;  // bit of the word's first offset for even pixels; -3 or more
+          const unsigned even = (unsigned)(i0 >= 0 ? bits >> i0 : bits << -i0) & 15u;
+          const unsigned odd = (unsigned)(i0 >= 1 ? bits >> (i0 - 1) : bits << (1 - i0)) & 15u;
+          if (!(even | odd)) {
+            loaded = false;
+            continue;
+          }
 #pragma unroll
-        for (int j = 0; j < kRowsPerWarp; ++j) {
-          const uint32_t* row = S + (j0 + j + kr) * kRowWords;
-          for (uint64_t m = bits; m; m &= m - 1) {
-            const int s = __ffsll((long long)m) - 1 - bw;
-            acc[j].odd = fold<MAX>(acc[j].odd, word_at(row, lane, s));
-            acc[j].even = fold<MAX>(acc[j].even, word_at(row, lane, s - 1));
+          for (int j = 0; j < kRowsPerWarp; ++j) {
+            cur[j] = loaded ? next[j] : row[j * kRowWords + wd];
+            next[j] = row[j * kRowWords + wd + 1];
+          }
+          loaded = true;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (!(((even | odd) >> q) & 1u)) continue;
+            uint32_t w[kRowsPerWarp];
+#pragma unroll
+            for (int j = 0; j < kRowsPerWarp; ++j) w[j] = q ? __funnelshift_r(cur[j], next[j], 8 * q) : cur[j];
+            if ((odd >> q) & 1u) {
+#pragma unroll
+              for (int j = 0; j < kRowsPerWarp; ++j) acc[j].odd = fold<MAX>(acc[j].odd, w[j]);
+            }
+            if ((even >> q) & 1u) {
+#pragma unroll
+              for (int j = 0; j < kRowsPerWarp; ++j) acc[j].even = fold<MAX>(acc[j].even, w[j]);
+            }
           }
         }
       }
@@ -279,10 +303,12 @@ __global__ void __launch_bounds__(kThreads, 2) morph_kernel(const uint8_t* __res
   }
 }
 
-// Staged rows, and the four planes of the centred path.
+// Staged rows, and the planes of the centred path: four, or as many as there are radii above 0 (the 3 x 3
+// elements then need no more than the 48 KB that a launch has without asking).
 size_t morph_smem(const MorphElement& e) {
   const size_t rows_in = kTileRows + 2 * (size_t)e.bw;
-  return sizeof(uint32_t) * rows_in * (kRowWords + (e.centred ? kGroup * kTileWords : 0));
+  const size_t planes = e.centred ? (e.max_radius < 1 ? 1 : e.max_radius < kGroup ? e.max_radius : kGroup) : 0;
+  return sizeof(uint32_t) * rows_in * (kRowWords + planes * kTileWords);
 }
 
 bool words_ok(const void* p, int64_t pitch) { return ((uintptr_t)p % 4) == 0 && pitch % 4 == 0; }
@@ -340,17 +366,16 @@ cudaError_t morph_open_launch(const uint8_t* in, int64_t pitch_in, uint8_t* out,
   const int tiles_y = (rows + kTileRows - 1) / kTileRows;
   const dim3 grid((cols + 4 * kTileWords - 1) / (4 * kTileWords), tiles_y < 65535 ? tiles_y : 65535);
   const size_t smem = morph_smem(e);
+  const auto erode = e.centred ? morph_kernel<false, true> : morph_kernel<false, false>;
+  const auto dilate = e.centred ? morph_kernel<true, true> : morph_kernel<true, false>;
   if (smem > 48 * 1024) {
-    cudaError_t r = cudaFuncSetAttribute(morph_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (r == cudaSuccess)
-      r = cudaFuncSetAttribute(morph_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t r = cudaFuncSetAttribute(erode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (r == cudaSuccess) r = cudaFuncSetAttribute(dilate, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (r != cudaSuccess) return r;
   }
-  morph_kernel<false><<<grid, kThreads, smem, s>>>(in, pitch_in, words_ok(in, pitch_in), quads_ok(in, pitch_in), tmp,
-                                                   pitch_tmp, true, rows,
-                                                   cols, e);
-  morph_kernel<true><<<grid, kThreads, smem, s>>>(tmp, pitch_tmp, true, true, out, pitch_out, words_ok(out, pitch_out),
-                                                  rows, cols, e);
+  erode<<<grid, kThreads, smem, s>>>(in, pitch_in, words_ok(in, pitch_in), quads_ok(in, pitch_in), tmp, pitch_tmp, true,
+                                     rows, cols, e);
+  dilate<<<grid, kThreads, smem, s>>>(tmp, pitch_tmp, true, true, out, pitch_out, words_ok(out, pitch_out), rows, cols, e);
   return cudaGetLastError();
 }
 
