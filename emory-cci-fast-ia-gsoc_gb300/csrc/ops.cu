@@ -1854,7 +1854,8 @@ __device__ __forceinline__ float fix_to_float(unsigned long long lo, long long h
 // Sources are near their pixels (a plateau grows a few pixels around its source), so the sums are
 // formed per 32 x 32 tile in shared memory by the CTA that owns the sources, and only pixels whose
 // source lies in another tile go through 128-bit accumulators in the workspace:
-//   (1) grad_touch: the accumulators such pixels use are zeroed and marked in a bitmap;
+//   (1) grad_touch: the accumulators such pixels use are zeroed and marked in a bitmap (a small image has
+//       all of them zeroed by the first launch instead, and (2) does the marking);
 //   (2) grad_far: such pixels add to them (two 64-bit atomics each, runs of one row summed first);
 //   (3) grad_tiles: every tile sums its own pixels, adds the marked accumulators, rounds, writes;
 //   (4) grad_wide_tiles: the same for tiles whose gradients span too many bits for (3).
@@ -1936,7 +1937,10 @@ __global__ void __launch_bounds__(128) grad_touch_kernel(GradArgs a) {
 // (low word, then the high word with the low word's carry).  Four rows per thread, their sources
 // loaded together; a warp without a far pixel in a row skips the row.
 constexpr int kFarRows = 4;
+template <bool MARK>
 __global__ void __launch_bounds__(128) grad_far_kernel(GradArgs a) {
+  pdl_wait();
+  pdl_release();
   const int lane = threadIdx.x & 31;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   for (int img = blockIdx.z; img < a.n; img += gridDim.z) {
@@ -1974,7 +1978,9 @@ __global__ void __launch_bounds__(128) grad_far_kernel(GradArgs a) {
         }
         const bool tail = lane == 31 || knext != key;
         if (tail && key >= 0) {
-          unsigned long long* q = a.acc[key >> 40] + 2 * (key & ((1ll << 40) - 1));
+          const int64_t gq = key & ((1ll << 40) - 1);
+          unsigned long long* q = a.acc[key >> 40] + 2 * gq;
+          if (MARK) atomicOr(a.far_bits[key >> 40] + (gq >> 5), 1u << (gq & 31));
           const unsigned long long old = atomicAdd(q, v.lo);
           const unsigned long long carry = old + v.lo < old ? 1ull : 0ull;
           atomicAdd(q + 1, (unsigned long long)v.hi + carry);
@@ -2010,17 +2016,18 @@ __device__ __forceinline__ Fix128 far_sum(const GradArgs& a, int c, int64_t gq) 
   return Fix128{v.x, (long long)v.y};
 }
 
-// When the tile's non-zero gradients lie within 30 binary orders of magnitude (and above 2^-73,
-// where every bit counts), each is an integer of 53 bits at most in units of the smallest one's last
-// bit, and the sum of all 1024 fits 63 bits.  It is added to three signed 32-bit limbs of 21 bits
-// (1024 pixels cannot overflow one) without returning atomics or carries, and the total converts
-// to float with one rounding (the scale is a power of two).  Tiles outside that range are listed
-// for grad_wide_tiles.
+// When the tile's non-zero gradients lie within 30 binary orders of magnitude, counted from 2^-73 at
+// least (where the last of 24 bits is the resolution, 2^-96), each is an integer of 53 bits at most in units
+// of the smallest one's last bit or of the resolution, to which it is rounded as in the wide sums, and the
+// sum of all 1024 fits 63 bits.  It is added to three signed 32-bit limbs of 21 bits (1024 pixels cannot
+// overflow one) without returning atomics or carries, and the total converts to float with one
+// rounding (the scale is a power of two).  Tiles outside that range are listed for grad_wide_tiles.
 constexpr int kSpan = 29;
 struct alignas(16) GradLimbs {  // cleared 16 bytes at a time
   int v[2][3][kGradPx];
 };
 static_assert(alignof(GradLimbs) >= alignof(uint4) && sizeof(GradLimbs) % sizeof(uint4) == 0, "cleared as uint4");
+constexpr int kUnitEx = 127 - 73;  // exponent whose last bit is the resolution
 __global__ void __launch_bounds__(kGradThreads) grad_tiles_kernel(GradArgs a) {
   __shared__ GradLimbs limbs;
   int (&limb)[2][3][kGradPx] = limbs.v;
@@ -2053,7 +2060,9 @@ __global__ void __launch_bounds__(kGradThreads) grad_tiles_kernel(GradArgs a) {
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < kGradThreads / 32; ++w) lo = min(lo, s_lo[w]), hi = max(hi, s_hi[w]);
-  if (lo <= hi && (lo < 127 - 73 || hi >= 127 + 31 || hi - lo > kSpan)) {
+  const bool below = lo < kUnitEx;  // the same for the whole tile
+  lo = max(lo, kUnitEx);
+  if (hi >= 127 + 31 || hi - lo > kSpan) {
     if (threadIdx.x == 0) a.wide[1 + atomicAdd(a.wide, 1)] = blockIdx.x;
     return;
   }
@@ -2067,7 +2076,16 @@ __global__ void __launch_bounds__(kGradThreads) grad_tiles_kernel(GradArgs a) {
     }
     if (other_tile(s, yw + k, x) || (g[k] << 1) == 0u) continue;
     const int i = (s.y & (kGradTile - 1)) * kGradTile + (s.x & (kGradTile - 1));
-    const unsigned long long v = (unsigned long long)((g[k] & 0x7FFFFFu) | 0x800000u) << (((g[k] >> 23) & 0xFF) - lo);
+    const int ex = (g[k] >> 23) & 0xFF;
+    unsigned long long v = (g[k] & 0x7FFFFFu) | 0x800000u;
+    if (!below || ex >= lo) {
+      v <<= ex - lo;
+    } else {  // below the resolution (lo = kUnitEx): nearest, ties to even; far below it nothing is left
+      const int r = lo - ex;
+      const unsigned m = (unsigned)v, rem = r < 32 ? m & ((1u << r) - 1u) : 0u, half = 1u << (min(r, 32) - 1);
+      const unsigned q = r < 32 ? m >> r : 0u;
+      v = q + ((rem > half || (rem == half && (q & 1u))) ? 1u : 0u);
+    }
     const int sign = (int)g[k] >> 31;  // 0 or -1
     constexpr int kMask = (1 << 21) - 1;
     const int l0 = (int)v & kMask, l1 = (int)(v >> 21) & kMask, l2 = (int)(v >> 42);
@@ -2103,7 +2121,7 @@ __global__ void __launch_bounds__(kGradThreads) grad_tiles_kernel(GradArgs a) {
     }
   }
   __syncthreads();
-  const int up = lo <= hi ? lo - 150 + 96 : 0;  // the tile's unit is 2^(up - 96), 0 <= up <= 103
+  const int up = hi ? lo - kUnitEx : 0;  // the tile's unit is 2^(up - 96), 0 <= up <= 103
   for (int j = threadIdx.x; j < listed; j += kGradThreads) {
     const int c = list[j] / kGradPx, i = list[j] & (kGradPx - 1);
     const int y = T.y0 + i / kGradTile, xi = T.x0 + (i & (kGradTile - 1));
@@ -2121,22 +2139,25 @@ __global__ void __launch_bounds__(kGradThreads) grad_tiles_kernel(GradArgs a) {
   }
 }
 
-// The listed tiles, any finite gradients below 2^31.  The first gradient a source receives stays in
-// its slot as it is; any further one is added to six signed 32-bit limbs of 21 bits (a gradient's
-// 24 bits touch three at most, and 1024 pixels cannot overflow the lower five).  Sources whose
-// limbs are not zero or that are marked in the bitmap are listed and converted densely; the others
-// are their slot.
-constexpr int kLimbs = 6, kLimbBits = 21;
-constexpr uint32_t kNoGrad = 0xFFFFFFFFu;  // a NaN: never a gradient in a slot
-struct alignas(16) GradTile {  // slots and limbs are set 16 bytes at a time
-  uint32_t slot[2][kGradPx];
-  int limb[2][kLimbs][kGradPx];
-  uint16_t list[2 * kGradPx];  // class * kGradPx + pixel
-  int listed;
+// The listed tiles, any finite gradients below 2^31.  Contributions are counted first.  The one gradient of
+// a source that gets no other stays as it is; the sources that get several (512 at most) have six signed
+// 32-bit limbs of 21 bits (a gradient's 24 bits touch three at most, and 1024 pixels cannot overflow the
+// lower five).  Sources with limbs or marked in the bitmap are listed and converted densely; the others are
+// their gradient.
+// Bound: latency at up to 48 warps an SM.  (A compare-and-swap per gradient for its source's slot, and limbs
+// for all 2048 sources -- 61 KB, three CTAs an SM -- took 82 us at 4 x 1024^2 with all tiles listed, this 68.)
+constexpr int kLimbs = 6, kLimbBits = 21, kMulti = kGradPx / 2;
+struct alignas(16) GradTile {  // counts and limbs are cleared 16 bytes at a time
+  int count[2 * kGradPx];      // class * kGradPx + pixel: gradients, or -1 - index of the limbs
+  int limb[kLimbs][kMulti];
+  uint32_t one[2 * kGradPx];   // the gradient where there is one
+  uint16_t list[2 * kGradPx];
+  int listed, multi;
 };
-static_assert(alignof(GradTile) >= alignof(uint4) && offsetof(GradTile, limb) % sizeof(uint4) == 0, "set as uint4");
+static_assert(alignof(GradTile) >= alignof(uint4) && offsetof(GradTile, limb) % sizeof(uint4) == 0, "cleared as uint4");
+constexpr int kWideCtasPerSm = 6;  // shared memory
 
-__device__ __forceinline__ void limb_add(int (*limb)[kGradPx], int i, float g) {
+__device__ __forceinline__ void limb_add(int (*limb)[kMulti], int i, float g) {
   const uint32_t b = __float_as_uint(g), ex = (b >> 23) & 0xFFu;
   uint32_t man = b & 0x7FFFFFu;
   int s = ex == 0 ? -149 + 96 : (int)ex - 150 + 96;  // g = +-man * 2^(s - 96)
@@ -2177,25 +2198,42 @@ __device__ __forceinline__ void grad_wide_tile(const GradArgs& a, GradTile& S, i
     p[k] = in ? __ldg(grad_row(a, a.prov, img, y) + x) : INT_MIN;
     g[k] = in ? __ldg(grad_row(a, a.g, img, y) + x) : 0.f;
   }
-  for (int i = threadIdx.x; i < 2 * kGradPx / 4; i += kGradThreads)
-    ((uint4*)S.slot)[i] = make_uint4(kNoGrad, kNoGrad, kNoGrad, kNoGrad);
-  for (int i = threadIdx.x; i < 2 * kLimbs * kGradPx / 4; i += kGradThreads)
-    ((uint4*)S.limb)[i] = make_uint4(0u, 0u, 0u, 0u);
-  if (threadIdx.x == 0) S.listed = 0;
+  for (int i = threadIdx.x; i < 2 * kGradPx / 4; i += kGradThreads) ((uint4*)S.count)[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = threadIdx.x; i < kLimbs * kMulti / 4; i += kGradThreads) ((uint4*)S.limb)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (threadIdx.x == 0) S.listed = S.multi = 0;
   __syncthreads();
+  int src[kRows];  // class * kGradPx + pixel of the tile's own sources, else -1
 #pragma unroll
   for (int k = 0; k < kRows; ++k) {
-    const int y = y0 + warp * kRows + k;
+    src[k] = -1;
     if (p[k] == INT_MIN) continue;
     const GradSource s = grad_source(a, p[k]);
-    const bool bad = (__float_as_uint(g[k]) & 0x7FFFFFFFu) >= (127u + 31u) << 23;  // |g| >= 2^31, inf, NaN
-    if (s.cls < 0 || bad) {
+    const uint32_t mag = __float_as_uint(g[k]) & 0x7FFFFFFFu;
+    if (s.cls < 0 || mag >= (127u + 31u) << 23) {  // |g| >= 2^31, inf, NaN
       set_status(a.status, NSGB_ERR_BAD_ARG);
       continue;
     }
-    if (other_tile(s, y, x)) continue;
-    const int i = (s.y & (kGradTile - 1)) * kGradTile + (s.x & (kGradTile - 1));
-    if (atomicCAS(&S.slot[s.cls][i], kNoGrad, __float_as_uint(g[k])) != kNoGrad) limb_add(S.limb[s.cls], i, g[k]);
+    if (mag == 0u || other_tile(s, y0 + warp * kRows + k, x)) continue;
+    src[k] = s.cls * kGradPx + (s.y & (kGradTile - 1)) * kGradTile + (s.x & (kGradTile - 1));
+    atomicAdd(&S.count[src[k]], 1);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * kGradPx; i += kGradThreads) {  // whole warps
+    const bool many = S.count[i] > 1;
+    const unsigned m = __ballot_sync(NSGB_FULL, many);
+    if (!m) continue;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&S.multi, __popc(m));
+    base = __shfl_sync(NSGB_FULL, base, 0);
+    if (many) S.count[i] = -1 - (base + __popc(m & ((1u << lane) - 1u)));
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kRows; ++k) {
+    if (src[k] < 0) continue;
+    const int n = S.count[src[k]];
+    if (n > 0) S.one[src[k]] = __float_as_uint(g[k]);
+    else limb_add(S.limb, -1 - n, g[k]);
   }
   __syncthreads();
 #pragma unroll
@@ -2203,53 +2241,51 @@ __device__ __forceinline__ void grad_wide_tile(const GradArgs& a, GradTile& S, i
     float* const out = c ? a.dmask : a.dmarker;
 #pragma unroll
     for (int k = 0; k < kRows; ++k) {
-      const int i = (warp * kRows + k) * kGradTile + lane;
+      const int i = c * kGradPx + (warp * kRows + k) * kGradTile + lane;
       const int y = y0 + warp * kRows + k;
       const bool in = y < a.H && x < a.W;
-      int any = 0;
-#pragma unroll
-      for (int l = 0; l < kLimbs; ++l) any |= S.limb[c][l][i];
-      const uint32_t first = S.slot[c][i];
-      bool more = any != 0;
+      bool more = false;
       if (in) {
-        const int64_t gq = px0 + (int64_t)y * a.W + x;
-        more = more || far_marked(a, c, gq);
+        const int n = S.count[i];
+        const uint32_t one = n > 0 ? S.one[i] : 0u;
         // a gradient below 2^-73 still has to be rounded to the resolution
-        const uint32_t mag = first == kNoGrad ? 0u : first & 0x7FFFFFFFu;
-        if (mag != 0u && mag < (127u - 73u) << 23) more = true;
-        if (!more) grad_row(a, out, img, y)[x] = mag == 0u ? 0.f : __uint_as_float(first);
+        more = n < 0 || far_marked(a, c, px0 + (int64_t)y * a.W + x) ||
+               (n > 0 && (one & 0x7FFFFFFFu) < (uint32_t)kUnitEx << 23);
+        if (!more) grad_row(a, out, img, y)[x] = __uint_as_float(one);
       }
-      const unsigned m = __ballot_sync(NSGB_FULL, in && more);
+      const unsigned m = __ballot_sync(NSGB_FULL, more);
       if (m) {
         int base = 0;
         if (lane == 0) base = atomicAdd(&S.listed, __popc(m));
         base = __shfl_sync(NSGB_FULL, base, 0);
-        if (in && more) S.list[base + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(c * kGradPx + i);
+        if (more) S.list[base + __popc(m & ((1u << lane) - 1u))] = (uint16_t)i;
       }
     }
   }
   __syncthreads();
   for (int j = threadIdx.x; j < S.listed; j += kGradThreads) {
-    const int c = S.list[j] / kGradPx, i = S.list[j] & (kGradPx - 1);
+    const int c = S.list[j] / kGradPx, i = S.list[j] & (kGradPx - 1), n = S.count[S.list[j]];
     const int y = y0 + i / kGradTile, xi = T.x0 + (i & (kGradTile - 1));
-    __int128 sum = 0;
+    Fix128 v = {0ull, 0ll};
+    if (n < 0) {
+      __int128 sum = 0;
 #pragma unroll
-    for (int l = kLimbs - 1; l >= 0; --l) sum = sum * (1 << kLimbBits) + S.limb[c][l][i];
-    Fix128 v = {(unsigned long long)sum, (long long)(sum >> 64)};
-    const uint32_t first = S.slot[c][i];
-    Fix128 f;
-    if (first != kNoGrad && fix_from_float(__uint_as_float(first), f)) v = fix_add(v, f);
+      for (int l = kLimbs - 1; l >= 0; --l) sum = sum * (1 << kLimbBits) + S.limb[l][-1 - n];
+      v = Fix128{(unsigned long long)sum, (long long)(sum >> 64)};
+    } else if (n > 0) {
+      fix_from_float(__uint_as_float(S.one[S.list[j]]), v);
+    }
     const int64_t gq = px0 + (int64_t)y * a.W + xi;
     if (far_marked(a, c, gq)) v = fix_add(v, far_sum(a, c, gq));
     grad_row(a, c ? a.dmask : a.dmarker, img, y)[xi] = fix_to_float(v.lo, v.hi);
   }
 }
 
-__global__ void __launch_bounds__(kGradThreads) grad_wide_tiles_kernel(GradArgs a) {
-  extern __shared__ __align__(16) unsigned char grad_smem[];
+__global__ void __launch_bounds__(kGradThreads, kWideCtasPerSm) grad_wide_tiles_kernel(GradArgs a) {
+  __shared__ GradTile tile;
   const int n = __ldcg(a.wide);
   for (int j = blockIdx.x; j < n; j += gridDim.x) {
-    grad_wide_tile(a, *reinterpret_cast<GradTile*>(grad_smem), __ldcg(a.wide + 1 + j));
+    grad_wide_tile(a, tile, __ldcg(a.wide + 1 + j));
     __syncthreads();
   }
 }
@@ -2267,6 +2303,10 @@ size_t f32_fwd_bytes(int64_t batch, int64_t rows, int64_t cols) {
   const Plan P1 = single_plan(NSGB_F32, nullptr, nullptr, rows, cols, cols * 4);
   return ws_sizes(stacked_totals(P1.t, batch)).total;
 }
+
+// Up to this many pixels clearing all accumulators (32 bytes a pixel) is quicker than a launch that finds the
+// ones to clear (200 x 333: 2 against 5 us).
+constexpr size_t kGradSmallPx = 1 << 18;
 
 int64_t grad_tiles(int64_t batch, int64_t rows, int64_t cols) {
   return batch * ((rows + kGradTile - 1) / kGradTile) * ((cols + kGradTile - 1) / kGradTile);
@@ -2376,21 +2416,27 @@ nsgb_status nsgb_recon_f32_bwd(const float* grad_out, const int32_t* prov, float
   a.far_bits[1] = (unsigned*)(p + 256 + 2 * acc_bytes + bit_bytes);
   a.wide = (int*)(p + 256 + 2 * acc_bytes + 2 * bit_bytes);
   const bool vec = ((uintptr_t)prov % 16) == 0 && pitch % 16 == 0 && a.stride % 16 == 0;
-  cudaError_t e = cudaMemsetAsync(a.status, 0, sizeof(int), s);
-  // the bitmaps and the count of wide tiles behind them
-  if (e == cudaSuccess) e = cudaMemsetAsync(a.far_bits[0], 0, 2 * bit_bytes + sizeof(int), s);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(grad_wide_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradTile));
-  if (e == cudaSuccess) {
-    const unsigned gy = (unsigned)std::min<int64_t>(rows, 65535), gz = (unsigned)std::min<int64_t>(batch, 65535);
-    const dim3 quads((a.W + 511) / 512, gy, gz);
-    const dim3 rows4((a.W + 127) / 128, (unsigned)std::min<int64_t>((rows + kFarRows - 1) / kFarRows, 65535), gz);
-    const int64_t tiles = grad_tiles(batch, rows, cols);
+  const bool small = px <= kGradSmallPx;
+  // The first launch clears the status, the bitmaps, the count of wide tiles behind them and, for a small
+  // image, the accumulators in front of them.
+  unsigned* const first = small ? (unsigned*)a.acc[0] : a.far_bits[0];
+  const ccl::ZeroSpans z{{(unsigned*)a.status, first, nullptr, nullptr}, {1, (int)((unsigned*)a.wide - first) + 1, 0, 0}};
+  cudaError_t e = ccl::launch_k(false, ccl::zero_words, dim3(grid1d(z.total())), dim3(256), s, z);
+  const unsigned gy = (unsigned)std::min<int64_t>(rows, 65535), gz = (unsigned)std::min<int64_t>(batch, 65535);
+  const dim3 quads((a.W + 511) / 512, gy, gz);
+  const dim3 rows4((a.W + 127) / 128, (unsigned)std::min<int64_t>((rows + kFarRows - 1) / kFarRows, 65535), gz);
+  const int64_t tiles = grad_tiles(batch, rows, cols);
+  // (ordinary launches: the wait of a dependent one costs many short CTAs 20 us each at 16 x 2048^2)
+  if (e == cudaSuccess && !small) {
     if (vec) grad_touch_kernel<true><<<quads, 128, 0, s>>>(a);
     else grad_touch_kernel<false><<<quads, 128, 0, s>>>(a);
-    grad_far_kernel<<<rows4, 128, 0, s>>>(a);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess)
+    e = launch_dependent(small ? grad_far_kernel<true> : grad_far_kernel<false>, rows4, dim3(128), s, a);
+  if (e == cudaSuccess) {
     grad_tiles_kernel<<<(unsigned)tiles, kGradThreads, 0, s>>>(a);
-    grad_wide_tiles_kernel<<<(unsigned)std::min<int64_t>(tiles, 3 * 152), kGradThreads, sizeof(GradTile), s>>>(a);
+    grad_wide_tiles_kernel<<<(unsigned)std::min<int64_t>(tiles, kWideCtasPerSm * 152), kGradThreads, 0, s>>>(a);
     e = cudaGetLastError();
   }
   return finish(e, ws, s, opts);
