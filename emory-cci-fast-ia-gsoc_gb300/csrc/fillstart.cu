@@ -21,8 +21,6 @@
 // A level above the right one would leave the whole chain to do, and a level below it marks nothing, so
 // images without a level of their own have to be told from the others before anything is labelled.
 // The start is the plain marker when
-//   - border pixels are nearly always brighter than pixels inside: there every level inside is closed
-//     off, and the plain front is fast (one value);
 //   - the crops have no level (most pixels differ from all others), or the reaching levels are spread
 //     over many values (a slope, a vignette, a noise of many levels);
 //   - a band of rows across the image's middle, labelled first, is not reached from its ends (a wall
@@ -30,14 +28,16 @@
 //
 // What is tried is decided on the device, so every launch is made for every image.  The kernels of a level
 // that is not tried read one word and return: 52 us a level at 16384^2, 18 at 4096^2 (205 with a labelling
-// tile to a warp and a word read by every warp).  Times of the whole fill, u8 4-connected, plain front ->
-// this (start without the conditions above):
-//   31 noise levels, 16384^2 14.8 -> 5.0 ms (5.0), 4096^2 3.05 -> 0.69 (0.79), 1500 x 1400 0.65 -> 0.37 (0.53)
-//   1 px bright border, 16384^2 3.2 -> 2.3 ms (6.7), 4096^2 0.55 -> 0.47 (0.97), 1500 x 1400 0.23 -> 0.21 (0.49)
-//   bright surround, 16384^2 4.2 -> 3.5 ms (7.8), 4096^2 0.64 -> 0.62 (1.12), 1500 x 1400 0.28 -> 0.29 (0.59)
-//   closed wall 200 px in, 16384^2 3.3 -> 2.8 ms (8.7), 4096^2 0.59 -> 0.63 (1.12)
-// (The plain front itself is written four pixels at a time, faster than before, which pays for the
-// estimate; the wall at 4096^2 is the one kind found where that is not enough.)
+// tile to a warp and a word read by every warp).  Whole fill of u8 images, 4-connected, at 16384^2, 4096^2 and
+// 1500 x 1400, in ms from the plain front, and with this start:
+//   31 noise levels around dark objects     14.9  3.04 0.66    4.9  0.68 0.36
+//   dark noise, bright border of a pixel     3.2  0.55 0.23    2.0  0.28 0.14
+//   dark noise in a bright noisy surround    4.2  0.64 0.28    2.9  0.55 0.30
+//   flat dark ground, bright objects         3.3  0.57 0.24    2.0  0.30 0.16
+//   noise that rises along the image        11.0  1.46 0.68   10.1  1.33 0.63   (no level: plain marker)
+//   closed wall 200 px in                    3.3  0.59 0.39    2.7  0.63 0.36   (found by the band)
+// The plain marker itself is written four pixels at a time, which pays for the estimate (the front took
+// these times with a pixel at a time); the wall at 4096^2 is the one kind found where that is not enough.
 #include "fillstart.cuh"
 
 #include <limits.h>
@@ -62,11 +62,11 @@ constexpr int kTries = 3;
 constexpr int kCheckGrid = 64;   // check points per side
 constexpr int kCheckCtas = kCheckGrid * kCheckGrid / kThreads;
 static_assert(kCheckGrid * kCheckGrid % kThreads == 0, "whole CTAs");
-constexpr int kPairs = kCropThreads;  // border / inside pairs compared
 constexpr int kBandRows = 1024;  // rows of the band, at most an eighth of the image's
 constexpr int kUnitRows = 4;     // rows of 128 columns: what a warp writes of the start, or a multiple
 // Smaller sides keep the plain marker: 1024^2 u8 noise takes 0.61 ms from it and 0.59 from an estimated
-// start, 1300^2 u16 0.93 and 0.61, 768^2 u8 0.41 and 0.50.
+// start, 1300^2 u16 0.93 and 0.61, 768^2 u8 0.41 and 0.50 (measured with an estimate of 0.1 ms; this one
+// takes 0.035).
 constexpr int kMinSide = 1280;
 constexpr int64_t kSmallPx = 1 << 22;
 constexpr int kTilesPerRound = 1 << 16;  // labelling tiles for each round of a CTA: eight full loads of the device
@@ -112,24 +112,6 @@ struct AtMost {
   int level;
   __device__ uint32_t operator()(const Img& m, int y, int x) const { return value<T>(m, y, x) <= level ? 1u : 0u; }
 };
-
-// Point j of a grid of kPairs over the image.
-template <typename T>
-__device__ __forceinline__ int inside_value(const Img& m, int j) {
-  constexpr int kCols = 32, kRows = kPairs / kCols;
-  return value<T>(m, (int)(((int64_t)m.H * (2 * (j / kCols) + 1)) / (2 * kRows)),
-                  (int)(((int64_t)m.W * (2 * (j % kCols) + 1)) / (2 * kCols)));
-}
-
-// Whether border pixels are not nearly always brighter than pixels inside (the same for all CTAs); one
-// pair per thread.
-template <typename T>
-__device__ bool border_is_low(const Img& m) {
-  const int k = threadIdx.x;
-  int y, x;
-  ccl::border_pixel((int)(((int64_t)2 * (m.W + m.H) * k) / kPairs), m.H, m.W, y, x);
-  return __syncthreads_count(value<T>(m, y, x) <= inside_value<T>(m, (k * 181) % kPairs)) >= kPairs / 16;
-}
 
 __device__ __forceinline__ uint64_t shfl64(uint64_t v, int lane) {
   const uint32_t lo = __shfl_sync(NSGB_FULL, (uint32_t)v, lane), hi = __shfl_sync(NSGB_FULL, (uint32_t)(v >> 32), lane);
@@ -275,8 +257,7 @@ __device__ __forceinline__ int crop_level(const Img& m, int k, int* v) {
 }
 
 // The levels to try, `tries` at most, from the crops' conducting levels; one CTA, s: 6 * kCrops words.
-template <typename T>
-__device__ __forceinline__ void choose_levels(const Img& m, int tries, bool probe, FillCtl* c, int* s) {
+__device__ __forceinline__ void choose_levels(int tries, bool probe, FillCtl* c, int* s) {
   int* const own = s;                    // conducting levels
   int* const sorted = s + kCrops;        // ... in order
   int* const reach = s + 2 * kCrops;     // reaching levels
@@ -340,11 +321,10 @@ __device__ __forceinline__ void choose_levels(const Img& m, int tries, bool prob
     if (sorted[k] == middle) s_middle = rank;
     if (sorted[k] == upper) s_upper = rank;
   }
-  // A level above nearly all pixels is a rim's: what is inside fills evenly, and the plain front is fast.
-  const bool rim = __syncthreads_count(inside_value<T>(m, k) <= middle) > kPairs * 3 / 4;
+  __syncthreads();
   // One level has to reach most crops: with 31 noise levels the quartiles of the reaching levels lie one
   // level apart at most, with 256 two to four.
-  if (k != 0 || rim || middle == kNone || s_upper - s_middle > 1 || s_upper - s_lower > 2) return;
+  if (k != 0 || middle == kNone || s_upper - s_middle > 1 || s_upper - s_lower > 2) return;
   // A level just below the one that conducts is worth trying first where it reaches some way in: what it
   // marks starts lower (20 Mpixel i32, 8-connected: reconstruction 2144 us from the conducting level
   // alone, 535 with the level below).  The next level up is for a median that falls just short; one
@@ -369,7 +349,6 @@ __global__ void __launch_bounds__(kCropThreads) crop_kernel(const __grid_constan
   __shared__ int s[kCrop * (kCrop + 1)];
   static_assert(kCrop * (kCrop + 1) >= 6 * kCrops, "choose_levels");
   if (blockIdx.x == 0 && threadIdx.x == 0) *f.nroots = 0;
-  if (!border_is_low<T>(m)) return;  // all CTAs or none
   const int level = crop_level<T, CONN>(m, blockIdx.x, s);
   bool last = false;
   if (threadIdx.x == 0) {
@@ -378,7 +357,7 @@ __global__ void __launch_bounds__(kCropThreads) crop_kernel(const __grid_constan
     last = atomicAdd(&c->crops_done, 1) == kCrops - 1;
     __threadfence();
   }
-  if (__syncthreads_or(last)) choose_levels<T>(m, tries, probe, c, s);
+  if (__syncthreads_or(last)) choose_levels(tries, probe, c, s);
 }
 
 // Local pass of labelling `k`; its bits are cleared on the way.  A CTA takes `per` rounds of tiles that
