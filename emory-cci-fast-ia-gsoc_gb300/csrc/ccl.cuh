@@ -899,10 +899,10 @@ cudaError_t label_filled(const Cls& cls, const Imgs& I, const BatchTotals& t, in
 // block) are scratch.
 // Roots marked in `skip` (optional) are left out: not counted and not ranked.
 // With pdl, every launch is a programmatic dependent of the kernel before it (the caller's last
-// launch must be a kernel); with zeroed, `bits` and `counts` are already clear.
+// launch must be a kernel), and `bits` and `counts` are already clear.
 cudaError_t rank_roots(const Imgs& I, const BatchTotals& t, const Forest& f, int lo, int hi, int* rank,
                        unsigned* bits, size_t bits_bytes, int* block_tmp, int* wpre, int* counts, cudaStream_t s,
-                       const unsigned* skip = nullptr, bool pdl = false, bool zeroed = false);
+                       const unsigned* skip = nullptr, bool pdl = false);
 // The counts of rank_roots alone (no ranks), into `counts` that are already clear.  `bits` receives
 // the global roots' bits (scratch, not cleared first).
 cudaError_t count_roots(const Imgs& I, const BatchTotals& t, const Forest& f, int lo, int hi, unsigned* bits,

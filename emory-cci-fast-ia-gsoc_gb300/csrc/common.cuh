@@ -1,5 +1,5 @@
-// Shared device helpers: element traits for the packed compute words, bounded waits,
-// device status words, and the grid barrier used by the persistent kernels.
+// Shared device helpers: element traits for the packed compute words, the bound of waits, and
+// device status words.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -27,52 +27,10 @@ __device__ __forceinline__ void set_status(int* status, int code) {
   atomicCAS(status, 0, code);
 }
 
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned ld_acquire_u(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ int ld_relaxed(const int* p) {
   int v;
   asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-
-// Sense-free generation barrier over all CTAs of a cooperative launch.  `bar[0]` counts
-// arrivals, `bar[1]` is the generation.  Returns false (and sets the status) if a wait timed
-// out; the caller then leaves its loop.
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, int* status) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s_ok = 1;
-    unsigned gen = ld_acquire_u(bar + 1);
-    __threadfence();
-    unsigned arrived = atomicAdd(bar, 1u) + 1u;
-    if (arrived == nblocks) {
-      atomicExch(bar, 0u);
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      long long spins = 0;
-      while (ld_acquire_u(bar + 1) == gen) {
-        if (++spins > kSpinLimit) {
-          set_status(status, kDevTimeout);
-          s_ok = 0;
-          break;
-        }
-        __nanosleep(256);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return s_ok != 0;
 }
 
 // ---------------------------------------------------------------------------------------

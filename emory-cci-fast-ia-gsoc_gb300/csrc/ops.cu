@@ -926,7 +926,7 @@ cudaError_t chain_impl(int dtype, const Plan& P, const Ws& w, int recon_conn, do
     // From the labelling on, every launch is a programmatic dependent of the one before it.
     if (e == cudaSuccess)
       e = ccl::rank_roots(P.I, t, w.forest(true), area_min, area_max, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre,
-                          w.counts, s, outside, true, true);
+                          w.counts, s, outside, true);
     if (e == cudaSuccess) {
       const int64_t W1 = P.I.d ? 0 : P.I.one.W;
       e = launch_dependent(label_out_kernel<true, true, true>, qrb(t), dim3(256), s, P.I, t.rows, (const int*)w.L,
@@ -962,7 +962,7 @@ cudaError_t chain_impl(int dtype, const Plan& P, const Ws& w, int recon_conn, do
     }
     if (e == cudaSuccess)
       e = ccl::rank_roots(P.I, t, w.forest(true), area_min, area_max, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre,
-                          w.counts, s, nullptr, true, true);
+                          w.counts, s, nullptr, true);
     if (e == cudaSuccess)
       e = launch_dependent(label_line_kernel<true, true, true>, dim3((t.blocks + kLineBlocks - 1) / kLineBlocks),
                            dim3(ccl::kBlockPx / 4), s, P.I, t.blocks, (const int*)w.L, (const int*)w.R,
@@ -1308,7 +1308,7 @@ nsgb_status nsgb_bwlabel(const uint8_t* bin, int32_t* labels, int64_t rows, int6
   cudaError_t e = ccl::label(ClsValueU8{}, P.I, P.t, conn, w.forest(false), s, call_spans(w, true, 2));
   if (e == cudaSuccess)
     e = ccl::rank_roots(P.I, P.t, w.forest(false), 0, 0, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre, w.counts, s, nullptr,
-                        true, true);
+                        true);
   if (e == cudaSuccess)
     e = launch_dependent(relabel ? label_out_kernel<true, false> : label_out_kernel<false, false>, qr(rows, cols),
                          dim3(256), s, P.I, P.t.rows, (const int*)w.L, (const int*)w.R, labels, pitch_labels,
@@ -1336,7 +1336,7 @@ nsgb_status nsgb_bwareaopen(const void* in, int labeled, int32_t* labels_out, ui
     e = ccl::label(ClsValueU8{}, P.I, P.t, conn, w.forest(true), s, call_spans(w, true, 2));
     if (e == cudaSuccess)
       e = ccl::rank_roots(P.I, P.t, w.forest(true), min_size, max_size, w.R, w.bits, w.bits_bytes, w.tmp, w.wpre, w.counts,
-                          s, nullptr, true, true);
+                          s, nullptr, true);
     if (e == cudaSuccess)
       e = launch_dependent(label_out_kernel<false, true>, qr(rows, cols), dim3(256), s, P.I, P.t.rows, (const int*)w.L,
                            (const int*)w.R, (int32_t*)nullptr, (int64_t)0, (const int*)w.A, min_size, max_size, labels_out,

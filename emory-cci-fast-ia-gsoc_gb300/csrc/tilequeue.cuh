@@ -20,8 +20,10 @@ struct alignas(8) Slot {
   unsigned seq;
 };
 
-// One 64-bit word, changed by one atomic: `pending` in the low half (never negative, never above
-// the number of tiles, so nothing carries into the upper half), the ticket counter above it.
+// One 64-bit word, changed by one atomic: `pending` in the low half, the ticket counter above it.
+// `pending` is never negative and at most twice the number of tiles (a tile given up by `and ~2` can be
+// marked and counted again before its own release is counted), far below 2^32: nothing carries into
+// the upper half.
 struct alignas(8) Tally {
   int pending;
   unsigned tail;
