@@ -645,6 +645,12 @@ void canon_zero(void* out, int64_t rows, int64_t cols, int64_t pitch, cudaStream
 // per pixel took 49 us at 4096^2 f32).
 template <typename T>
 using HminH = std::conditional_t<std::is_floating_point<T>::value, T, int64_t>;
+// (Within 62 bits: a conversion beyond the type is undefined, and the sum with a pixel has to fit.  NaN is no h.)
+template <typename T>
+HminH<T> hmin_h(double h) {
+  if constexpr (std::is_floating_point<T>::value) return (T)h;
+  else return h != h ? 0 : (int64_t)std::min(std::max(h, -0x1p62), 0x1p62);
+}
 template <typename T>
 __device__ __forceinline__ T hmin_value(T v, HminH<T> h) {
   if constexpr (std::numeric_limits<T>::is_integer) {
@@ -1252,7 +1258,7 @@ nsgb_status nsgb_imhmin(int dtype, const void* image, void* out, int64_t rows, i
   const bool vec = ((uintptr_t)image % (4 * esz)) == 0 && ((uintptr_t)out % (4 * esz)) == 0 && pitch % (4 * esz) == 0;
   dispatch_all(dtype, [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
-    const auto hh = (HminH<T>)h;
+    const auto hh = hmin_h<T>(h);
     if (vec) hmin_marker_kernel<T, true><<<quad_grid(rows, cols), 256, 0, s>>>((const T*)image, (T*)out, pitch, H, W, hh);
     else hmin_marker_kernel<T, false><<<quad_grid(rows, cols), 256, 0, s>>>((const T*)image, (T*)out, pitch, H, W, hh);
   });

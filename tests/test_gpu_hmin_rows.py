@@ -40,3 +40,12 @@ def test_hmin_rows(nsgb, oracle, dtype, w):
             exp = oracle.imhmin(host, 3.0, conn)
             assert np.array_equal(body[:, :w].view(f"u{item}"), np.asarray(exp, dtype).view(f"u{item}")), (pitch, conn)
             assert (body[:, w:] == 7).all() and (got[:off_out] == 7).all() and (got[off_out + h * pitch:] == 7).all()
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16])
+@pytest.mark.parametrize("h", [1e18, 9.3e18, 1e30, float("inf")])
+def test_hmin_beyond_the_type(nsgb, oracle, dtype, h):
+    """An h above every pixel, in and beyond 64 bits, is the largest h of the type."""
+    img = np.random.default_rng(3).integers(0, 200, (40, 61)).astype(dtype)
+    exp = oracle.imhmin(img, float(np.iinfo(dtype).max), 8)
+    assert np.array_equal(nsgb.imhmin(torch.from_numpy(img).cuda(), h, 8).cpu().numpy(), exp)
