@@ -68,7 +68,7 @@ constexpr int kUnitRows = 4;     // rows of 128 columns: what a warp writes of t
 // start, 1300^2 u16 0.93 and 0.61, 768^2 u8 0.41 and 0.50 (measured with an estimate of 0.1 ms; this one
 // takes 0.035).
 constexpr int kMinSide = 1280;
-constexpr int64_t kSmallPx = 1 << 22;
+constexpr int64_t kSmallPx = 1 << 23;
 constexpr int kTilesPerRound = 1 << 16;  // labelling tiles for each round of a CTA: eight full loads of the device
 
 // What is labelled: the image at level 0 .. kTries - 1, or the band at the highest of them.
@@ -78,7 +78,7 @@ constexpr int kBand = kTries;
 struct FillCtl {
   int go[kTries + 1];       // label it
   int level[kTries + 1];
-  int n, expected;          // levels, and which of them is the median reaching level
+  int n, expected;          // levels, and which of them is expected to conduct
   int low[kTries + 1];      // check points at or below the level
   int joined[kTries + 1];   // ... of them joined to the border
   int checked[kTries + 1];  // CTAs that have counted theirs
@@ -256,50 +256,57 @@ __device__ __forceinline__ int crop_level(const Img& m, int k, int* v) {
   return kNone;
 }
 
-// The levels to try, `tries` at most, from the crops' conducting levels; one CTA, s: 6 * kCrops words.
+// The levels to try, `tries` at most, from the crops' conducting levels; one CTA, s: 8 * kCrops words.
+// Reaching levels are taken over a crop's eight neighbours and over its four: a level that conducts
+// over any distance is crossed in more than half of the crops, between what it takes for most crops to be
+// reached over eight neighbours (41%, site percolation) and over four (59%).
 __device__ __forceinline__ void choose_levels(int tries, bool probe, FillCtl* c, int* s) {
   int* const own = s;                    // conducting levels
   int* const sorted = s + kCrops;        // ... in order
-  int* const reach = s + 2 * kCrops;     // reaching levels
-  int* const order = s + 3 * kCrops;     // ... in order
-  int* const distinct = s + 4 * kCrops;  // different conducting levels
-  int* const begin = s + 5 * kCrops;     // ... and the first crop in order of each
+  int* const distinct = s + 2 * kCrops;  // the different ones
+  int* const begin = s + 3 * kCrops;     // ... and the first crop in order of each
   __shared__ unsigned s_new[kCropWarps];
-  __shared__ int s_lower, s_middle, s_upper;
+  __shared__ int s_lower, s_middle, s_upper, s_expected;
   const int k = threadIdx.x;
   const bool crop = k < kCrops;
-  const int cy = k / kCropGrid, cx = k - cy * kCropGrid;
-  int mine = 0;
-  if (crop) {
-    own[k] = mine = __ldcg(&c->crop[k]);
-    reach[k] = cx == 0 || cx == kCropGrid - 1 ? mine : INT_MAX;
+  // threads 0 .. 143: eight neighbours, 256 .. 399: four
+  const int nb = k >> 8, i = k & 255;
+  const bool on = i < kCrops;
+  int* const reach = s + (4 + 2 * nb) * kCrops;  // reaching levels
+  int* const order = reach + kCrops;             // ... in order
+  const int cy = i / kCropGrid, cx = i - cy * kCropGrid;
+  int mine = 0, far = 0;
+  if (on) {
+    mine = __ldcg(&c->crop[i]);
+    if (nb == 0) own[i] = mine;
+    reach[i] = far = cx == 0 || cx == kCropGrid - 1 ? mine : INT_MAX;
   }
   if (__syncthreads_count(crop && mine == kNone) > kCrops / 4) return;
-  int far = crop ? reach[k] : 0;
   for (int it = 0; it < kCrops; ++it) {
     int r = INT_MAX;
-    if (crop) {
+    if (on) {
 #pragma unroll
       for (int d = 0; d < 9; ++d) {
         const int y = cy + d / 3 - 1, x = cx + d % 3 - 1;
+        if (nb == 1 && (d & 1) == 0 && d != 4) continue;
         if ((unsigned)y < (unsigned)kCropGrid && (unsigned)x < (unsigned)kCropGrid) r = min(r, reach[y * kCropGrid + x]);
       }
       r = max(r, mine);
     }
-    const bool lower = crop && r < far;
+    const bool lower = on && r < far;
     if (!__syncthreads_or(lower)) break;
-    if (lower) reach[k] = far = r;
+    if (lower) reach[i] = far = r;
     __syncthreads();
   }
-  if (crop) {
+  if (on) {
     int a = 0, b = 0;
 #pragma unroll 8
     for (int j = 0; j < kCrops; ++j) {
       const int o = own[j], r = reach[j];
-      a += o < mine || (o == mine && j < k);
-      b += r < far || (r == far && j < k);
+      a += o < mine || (o == mine && j < i);
+      b += r < far || (r == far && j < i);
     }
-    sorted[a] = mine;
+    if (nb == 0) sorted[a] = mine;
     order[b] = far;
   }
   __syncthreads();
@@ -313,27 +320,32 @@ __device__ __forceinline__ void choose_levels(int tries, bool probe, FillCtl* c,
     ranks += __popc(s_new[w]);
     if (w < (k >> 5)) rank += __popc(s_new[w]);
   }
-  const int lower = order[kCrops / 4], middle = order[kCrops / 2], upper = order[3 * kCrops / 4];
+  const int* const order8 = s + 5 * kCrops;
+  const int* const order4 = s + 7 * kCrops;
   if (fresh) {
-    distinct[rank] = sorted[k];
+    const int v = sorted[k];
+    distinct[rank] = v;
     begin[rank] = k;
-    if (sorted[k] == lower) s_lower = rank;
-    if (sorted[k] == middle) s_middle = rank;
-    if (sorted[k] == upper) s_upper = rank;
+    if (v == order8[kCrops / 4]) s_lower = rank;
+    if (v == order8[kCrops / 2]) s_middle = rank;
+    if (v == order8[3 * kCrops / 4]) s_upper = rank;
+    if (v == order4[kCrops / 2]) s_expected = rank;
   }
   __syncthreads();
   // One level has to reach most crops: with 31 noise levels the quartiles of the reaching levels lie one
   // level apart at most, with 256 two to four.
-  if (k != 0 || middle == kNone || s_upper - s_middle > 1 || s_upper - s_lower > 2) return;
-  // A level just below the one that conducts is worth trying first where it reaches some way in: what it
-  // marks starts lower (20 Mpixel i32, 8-connected: reconstruction 2144 us from the conducting level
-  // alone, 535 with the level below).  The next level up is for a median that falls just short; one
-  // that few crops hold is a wall's.
+  if (k != 0 || order4[kCrops / 2] == kNone || s_upper - s_middle > 1 || s_upper - s_lower > 2 ||
+      s_expected - s_middle > 1)
+    return;
+  // The level below the one that conducts is tried first although it does not reach the middle: what it
+  // marks starts lower, and without it the front near the border is the whole chain again (4096^2 i32,
+  // 8-connected, a level that reaches none of the inner half: 3.5 ms without, 1.3 with it).  The level above the expected one is for an estimate that falls just
+  // short; one that few crops hold is a wall's.
   int n = 0;
-  for (int r = s_middle - s_lower < tries ? s_lower : s_middle; r < ranks && r <= s_middle + 1 && n < tries; ++r) {
+  for (int r = s_expected - s_lower < tries ? s_lower : s_expected; r < ranks && r <= s_expected + 1 && n < tries; ++r) {
     const int held = (r + 1 < ranks ? begin[r + 1] : kCrops) - begin[r];
-    if (distinct[r] == kNone || (r > s_middle && held < kCrops / 8)) continue;
-    if (r == s_middle) c->expected = n;
+    if (distinct[r] == kNone || (r > s_expected && held < kCrops / 8)) continue;
+    if (r == s_expected) c->expected = n;
     c->level[n++] = distinct[r];
   }
   if (n == 0) return;
@@ -347,7 +359,7 @@ template <typename T, int CONN>
 __global__ void __launch_bounds__(kCropThreads) crop_kernel(const __grid_constant__ Img m, int tries, bool probe,
                                                             ccl::Forest f, FillCtl* c) {
   __shared__ int s[kCrop * (kCrop + 1)];
-  static_assert(kCrop * (kCrop + 1) >= 6 * kCrops, "choose_levels");
+  static_assert(kCrop * (kCrop + 1) >= 8 * kCrops && kCrops <= 256 && kCropThreads >= 512, "choose_levels");
   if (blockIdx.x == 0 && threadIdx.x == 0) *f.nroots = 0;
   const int level = crop_level<T, CONN>(m, blockIdx.x, s);
   bool last = false;
@@ -360,19 +372,16 @@ __global__ void __launch_bounds__(kCropThreads) crop_kernel(const __grid_constan
   if (__syncthreads_or(last)) choose_levels(tries, probe, c, s);
 }
 
-// Local pass of labelling `k`; its bits are cleared on the way.  A CTA takes `per` rounds of tiles that
-// follow one another.
+// Local pass of labelling `k`.  A CTA takes `per` rounds of tiles that follow one another.
 template <typename T, int CONN>
 __global__ void __launch_bounds__(32 * ccl::kLocalWarps)
-    local_kernel(const __grid_constant__ Img m, int ntiles, int per, int k, ccl::Forest f, unsigned* bits, int words,
-                 const FillCtl* c) {
+    local_kernel(const __grid_constant__ Img m, int ntiles, int per, int k, ccl::Forest f, const FillCtl* c) {
   pdl_wait();
   pdl_release();
   if (!active(c, k)) return;
   __shared__ int s_nodes[ccl::kLocalWarps][ccl::kTile * ccl::kTile];
   __shared__ unsigned s_starts[ccl::kLocalWarps][ccl::kTile];
   const AtMost<T> cls{__ldcg(&c->level[k])};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) bits[i] = 0u;
   const int warp = threadIdx.x >> 5;
   for (int i = 0; i < per; ++i) {
     const int b = (blockIdx.x * per + i) * ccl::kLocalWarps + warp;
@@ -382,13 +391,15 @@ __global__ void __launch_bounds__(32 * ccl::kLocalWarps)
   }
 }
 
+// Edge merge of labelling `k`; its bits are cleared on the way.
 template <typename T, int CONN>
 __global__ void __launch_bounds__(kThreads) merge_kernel(const __grid_constant__ Img m, int ntiles, int per, int k,
-                                                         ccl::Forest f, const FillCtl* c) {
+                                                         ccl::Forest f, unsigned* bits, int words, const FillCtl* c) {
   pdl_wait();
   pdl_release();
   if (!active(c, k)) return;
   const AtMost<T> cls{__ldcg(&c->level[k])};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) bits[i] = 0u;
   for (int i = 0; i < per; ++i) {
     const int e = (blockIdx.x * per + i) * kWarps + (threadIdx.x >> 5);
     if (e >= 2 * ntiles) break;
@@ -443,8 +454,9 @@ __device__ __forceinline__ void check_points(const Img& m, int k, const ccl::For
   if (k == kBand) {
     c->go[0] = 8 * joined >= low;
   } else if (k + 1 < __ldcg(&c->n)) {
-    // not when this level conducts, nor when it should have and marks next to nothing
-    c->go[k + 1] = low == 0 || (2 * joined < low && (k < __ldcg(&c->expected) || 16 * joined >= low));
+    // not when this level conducts, nor when it should have and marks next to nothing (unless the band says
+    // that the highest level does)
+    c->go[k + 1] = low == 0 || (2 * joined < low && (k < __ldcg(&c->expected) || 16 * joined >= low || __ldcg(&c->go[kBand])));
   }
 }
 
@@ -578,24 +590,23 @@ cudaError_t level_start(const Img& m, int c_tiles, const ccl::Forest& f, unsigne
                         cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(c, 0, sizeof(FillCtl), s);
   if (e != cudaSuccess) return e;
-  // Small images: no band, since labelling the whole costs little more than its launches (1500 x 1400 u8:
-  // band 40 us, level 85 us).
+  // Small images: no band, since labelling the whole costs little more (4096^2 u8: band 60 us, level 210).
   const bool probe = (int64_t)m.H * m.W > kSmallPx;
   const int tries = probe ? kTries : kTries - 1;
   crop_kernel<T, CONN><<<kCrops, kCropThreads, 0, s>>>(m, tries, probe, f, c);
   e = cudaGetLastError();
   const auto label = [&](const Img& img, int tiles, int nwords, int k) {
     // rounds per CTA: large images have fewer CTAs, which a level that is not tried starts for nothing
-    // (16384^2, local pass: 65536 CTAs take 1.11 ms, or 68 us to return at once; 16384 of four rounds 1.24
+    // (16384^2, local pass: 65536 CTAs take 1.20 ms, or 68 us to return at once; 16384 of four rounds 1.24
     // ms or 18 us; 1976 that take tiles in turn 1.42 ms)
     const int per = std::min(8, std::max(1, tiles / kTilesPerRound));
     const int warps = per * ccl::kLocalWarps, edges = per * kWarps;
     if (e == cudaSuccess)
       e = launch_dependent(local_kernel<T, CONN>, dim3((unsigned)((tiles + warps - 1) / warps)),
-                           dim3(32 * ccl::kLocalWarps), s, img, tiles, per, k, f, bits, nwords, (const FillCtl*)c);
+                           dim3(32 * ccl::kLocalWarps), s, img, tiles, per, k, f, (const FillCtl*)c);
     if (e == cudaSuccess)
       e = launch_dependent(merge_kernel<T, CONN>, dim3((unsigned)((2 * (int64_t)tiles + edges - 1) / edges)),
-                           dim3(kThreads), s, img, tiles, per, k, f, (const FillCtl*)c);
+                           dim3(kThreads), s, img, tiles, per, k, f, bits, nwords, (const FillCtl*)c);
     if (e == cudaSuccess)
       e = launch_dependent(mark_kernel<T>, dim3(ccl::list_grid((int64_t)img.H * img.W)), dim3(kThreads), s, img, k, f,
                            bits, (const FillCtl*)c);

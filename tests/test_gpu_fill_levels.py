@@ -57,8 +57,8 @@ def _fill(img, conn):
     return out.cpu().numpy(), [k for k in range(4) if go[k]]
 
 
-# sides of 1280, 2^22 pixels and one row more (where the band begins), a tall and a wide one
-@pytest.mark.parametrize("h,w", [(1280, 1283), (2048, 2048), (2049, 2048), (4500, 1281), (1290, 4127)])
+# sides of 1280, below and above 2^23 pixels (where the band begins), a tall and a wide one
+@pytest.mark.parametrize("h,w", [(1280, 1283), (2896, 2896), (2896, 2897), (4500, 1281), (1290, 6600)])
 @pytest.mark.parametrize("kind", ["noise", "frame", "rim", "surround", "slope", "many", "wall"])
 def test_levels_and_result(nsgb, oracle, kind, h, w):
     dtype = {"noise": np.int32, "surround": np.uint16}.get(kind, np.uint8)
@@ -70,5 +70,5 @@ def test_levels_and_result(nsgb, oracle, kind, h, w):
             assert 0 in tried, (conn, tried)
         elif kind in ("slope", "many"):
             assert tried == [], (conn, tried)
-        elif kind == "wall" and h * w > 1 << 22:
+        elif kind == "wall" and h * w > 1 << 23:
             assert tried in ([], [BAND]), (conn, tried)
