@@ -339,8 +339,8 @@ __device__ __forceinline__ void choose_levels(int tries, bool probe, FillCtl* c,
     return;
   // The level below the one that conducts is tried first although it does not reach the middle: what it
   // marks starts lower, and without it the front near the border is the whole chain again (4096^2 i32,
-  // 8-connected, a level that reaches none of the inner half: 3.5 ms without, 1.3 with it).  The level above the expected one is for an estimate that falls just
-  // short; one that few crops hold is a wall's.
+  // 8-connected, a level that reaches none of the inner half: 3.5 ms without, 1.3 with it).  The level
+  // above the expected one is for an estimate that falls just short; one that few crops hold is a wall's.
   int n = 0;
   for (int r = s_expected - s_lower < tries ? s_lower : s_expected; r < ranks && r <= s_expected + 1 && n < tries; ++r) {
     const int held = (r + 1 < ranks ? begin[r + 1] : kCrops) - begin[r];

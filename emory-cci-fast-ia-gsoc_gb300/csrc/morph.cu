@@ -24,7 +24,8 @@
 // one per plane, between two barriers), and the element rows of that radius fold the plane's rows
 // into the per-row accumulators.  A vertical run of eight or more element rows of one radius is a
 // sliding window: the rows common to a thread's eight outputs are folded once.
-// Other elements take the direct path: two folds (odd and even pixels) per element pixel.
+// Other elements, in a kernel of their own: two folds (odd and even pixels) per element pixel, of words
+// that the eight outputs of a thread and the two parities share.
 //
 // Bound: instructions issued.  4096^2 with the 19 x 19 disk: 49 us per pass at 66% of
 // issue cycles (the byte-wise form, one radius per barrier pair and 64-row tiles, took 102 us; this
